@@ -33,7 +33,8 @@ CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fvisibility=hid
             "-I", CSRC]
 
 # libpspw_gpu.so
-GPU_SOURCES = ["basis.cpp", "cell.cu", "hpsi.cu", "fftpath_f32.cu", "fftpath_f64.cu", "capi.cu",
+GPU_SOURCES = ["basis.cpp", "cell.cu", "hpsi.cu", "fftpath_f32.cu", "fftpath_f64.cu", "fftany_plane_f32.cu",
+               "fftany_plane_f64.cu", "fftany_sticks_f32.cu", "fftany_sticks_f64.cu", "capi.cu",
                "noalloc.cu", "gemm.cu", "heev.cu", "dense.cu", "solvers.cu", "capi_solvers.cu", "nl_tc.cu",
                "scf.cu", "scf_driver.cu", "input.cpp", "geom.cu", "serve.cpp", "batch.cu"]
 GPU_LIBS = ["-lcusolver", "-lcublas", "-lcudart"]
@@ -64,6 +65,8 @@ def _compile(src, force, headers):
         return obj, None
     if name.endswith(".cu"):
         cmd = [NVCC] + NVFLAGS + ["-c", src, "-o", obj]
+        if name.startswith("fftany"):  # many large kernels per file
+            cmd.insert(1, "--split-compile=3")
     else:
         cmd = ["g++"] + CXXFLAGS + ["-I", os.path.join(CUDA, "include"), "-c", src, "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -87,6 +90,8 @@ def build(force=False, jobs=8, verbose=True):
     errs = []
     objs = {}
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
+        # the longest compilations first
+        sources.sort(key=lambda s: not s.startswith("fftany"))
         futs = {ex.submit(_compile, os.path.join(CSRC, s), force, headers): s for s in sources}
         for f in cf.as_completed(futs):
             obj, err = f.result()

@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "fftpath.h"
 
 namespace pspw {
 namespace {
@@ -91,7 +92,7 @@ int chebyfilt_dev(pspw_cell *c, void *Xv, int ld, int ngw, int nb, int degree, d
   // the cell's stick-order arrays swapped in (contiguous stick gathers and
   // scatters), and the result is permuted back.  The recurrence is the same
   // arithmetic on the same numbers in another order of G.
-  const bool stick = c->basis.fast && ngw == c->basis.ngw;
+  const bool stick = fast_path<R>(c->basis) && ngw == c->basis.ngw;
   T *X0 = X;
   int ld0 = ld;
   if (stick) {

@@ -102,7 +102,7 @@ int eval_rho_psi_dev(pspw_cell *c, const double2 *dX, int ld, int ngw, int nx, c
   PSPW_CUDA(cudaMemcpyAsync(dw, wband.data(), sizeof(double) * nx, cudaMemcpyHostToDevice, c->stream));
   k_charge_sums<<<nx, 256, 0, c->stream>>>(dX, ld, m, B.d_xkg64, dsum, dsum + nx);
   c->kernel_launches++;
-  if (B.fast) {
+  if (B.fast_rho) {
     const FastGeo g{B.ncol,    B.nxa,       B.d_col_start, B.d_sg_ig,
                     B.d_sg_z,  B.d_sg_col,  B.d_xa_list,   B.d_col_x,
                     B.d_col_y, B.d_xa_of_x, false,         B.d_sg_off};

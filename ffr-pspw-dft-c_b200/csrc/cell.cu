@@ -402,8 +402,8 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
     sg_ig[k] = ig;
     sg_z[k] = gi3[ig];
     sg_col[k] = col_of_xy[(size_t)gi1[ig] + (size_t)nr1 * gi2[ig]];
-    // below 2^16 on every compiled length (at most 16 x 129); the generic
-    // path does not read it
+    // below 2^16 on every length of the register path (tile x (n3 + 1));
+    // the generic path does not read it
     sg_off[k] = (unsigned short)std::min(65535, (sg_col[k] % tile) * (nr3 + 1) + sg_z[k]);
   }
   std::vector<int> xa_of_x(nr1, -1), xa_list;
@@ -436,13 +436,13 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
   for (int i = 0; i < 3; i++)
     if ((rc = make_dim(B.dim[i], nr[i]))) return bail(rc);
   // register-FFT path when all three lengths split into two register DFTs
-  B.fast = !std::getenv("PSPW_GENERIC_FFT") && fast_supported(nr1, nr2, nr3);
-  if (B.fast) {
+  set_fft_paths(&B);
+  if (B.fast32) {
     if ((rc = upload(&B.d_col_x, col_x)) || (rc = upload(&B.d_col_y, col_y))) return bail(rc);
     for (int i = 0; i < 3; i++) {
-      const NSplit sp = nsplit_for(nr[i]);
+      const Split &sp = B.split[i];
       std::vector<int> pinv(nr[i]);
-      for (int p = 0; p < nr[i]; p++) pinv[p] = p / sp.n1 + sp.n2 * (p % sp.n1);
+      for (int p = 0; p < nr[i]; p++) pinv[p] = p / sp.a + sp.b * (p % sp.a);
       if ((rc = upload(&B.d_pinv[i], pinv))) return bail(rc);
     }
     if (cudaMalloc(&c->d_vperm64, (size_t)B.nnr * sizeof(double)) != cudaSuccess ||
@@ -639,7 +639,7 @@ int pspw_cell_set_veff_device(pspw_cell *c, const double *d_veff, int nnr) {
                                                 c->d_veff32);
   c->kernel_launches++;
   const Basis &B = c->basis;
-  if (B.fast) {
+  if (B.fast32) {
     k_veff_perm<<<2 * 148, 256, 0, c->stream>>>(d_veff, B.n1, B.n2, B.n3, 1.0 / (double)nnr,
                                                  B.d_pinv[0], B.d_pinv[1], B.d_pinv[2],
                                                  c->d_vperm64, c->d_vperm32);

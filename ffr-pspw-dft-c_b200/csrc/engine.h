@@ -23,6 +23,12 @@ struct FftDim {
   float2 *d_w32 = nullptr;
 };
 
+// A grid length as block factor x strided factor of the register FFT (a == 0:
+// no split).
+struct Split {
+  int n = 0, a = 0, b = 0;
+};
+
 // Device copy of the basis in the layouts the kernels read.
 //
 // The wavefunction sphere is organised in "sticks": the distinct (i1,i2)
@@ -49,10 +55,13 @@ struct Basis {
   double *d_xkg64 = nullptr;   // [ngw] XKG (the preconditioner and EKIN read it)
   int *d_wgrid = nullptr;      // [ngw] 0-based grid index of G (N123 - 1)
   FftDim dim[3];
-  // register-FFT path (every length has a two-factor split): stick
-  // coordinates, and per axis the natural index held at each position of
-  // the digit-permuted order
-  bool fast = false;
+  // register-FFT path (every length has a two-factor split and the plane of
+  // the precision fits in shared memory): the splits, stick coordinates, and
+  // per axis the natural index held at each position of the digit-permuted
+  // order
+  bool fast32 = false, fast64 = false;
+  bool fast_rho = false;  // the FP64 plane and its density accumulator fit
+  Split split[3];
   int *d_col_x = nullptr;  // [ncol]
   int *d_col_y = nullptr;  // [ncol]
   int *d_pinv[3] = {nullptr, nullptr, nullptr};

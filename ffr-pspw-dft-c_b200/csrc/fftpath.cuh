@@ -434,10 +434,13 @@ int rho_fast(pspw_cell *c, const FastGeo &g, const cx<R> *psi, int ld, int ngw_s
     const int nbb = std::min(nbatch, nb - b0);
     const int bpg = (nbb + ngroups - 1) / ngroups;
     const int ng = (nbb + bpg - 1) / bpg;
-    rc = dispatch_sticks_inv<T>(B.n3, g, st, nbb, wz, psi + (size_t)b0 * ld, ld, ngw_scatter, S);
-    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "density: length not compiled") : rc;
+    const T *pb = psi + (size_t)b0 * ld;
+    rc = dispatch_sticks_inv<T>(B.n3, g, st, nbb, wz, pb, ld, ngw_scatter, S);
+    if (rc < 0) rc = any_sticks_inv<T>(B, g, st, nbb, wz, pb, ld, ngw_scatter, S);
+    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "density: no kernel for this length") : rc;
     rc = dispatch_plane_rho<T>(B.n1, B.n2, g, st, B.n3, ng, wx, wy, S, nbb, bpg, d_wband + b0, part);
-    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "density: plane not compiled") : rc;
+    if (rc < 0) rc = any_plane_rho<T>(B, g, st, ng, wx, wy, S, nbb, bpg, d_wband + b0, part);
+    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "density: no kernel for this plane") : rc;
     k_rho_reduce<<<2 * 148, 256, 0, st>>>(part, ng, B.n1, B.n2, B.n3, B.d_pinv[0], B.d_pinv[1],
                                            B.d_pinv[2], d_rho);
     c->kernel_launches += 3;
@@ -483,22 +486,27 @@ int local_fast(pspw_cell *c, const FastGeo &g, const cx<R> *in, int ld_in, cx<R>
     int rc;
     timing_begin(c, kFamSticksInv, &e2);
     rc = dispatch_sticks_inv<T>(B.n3, g, st, nbb, wz, inb, ld_in, ngw, S);
+    if (rc < 0) rc = any_sticks_inv<T>(B, g, st, nbb, wz, inb, ld_in, ngw, S);
     timing_end(c, kFamSticksInv, e2);
     c->kernel_launches++;
-    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: length not compiled") : rc;
+    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: no kernel for this length") : rc;
     timing_begin(c, kFamXlines, &e2);
     rc = dispatch_plane<T, R>(B.n1, B.n2, g, st, nbb, B.n3, wx, wy, PrecF<R>::vperm(c), S);
+    if (rc < 0) rc = any_plane<T, R>(B, g, st, nbb, wx, wy, PrecF<R>::vperm(c), S);
     timing_end(c, kFamXlines, e2);
     c->kernel_launches++;
-    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: plane not compiled") : rc;
+    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: no kernel for this plane") : rc;
     timing_begin(c, kFamSticksFwd, &e2);
     RecArg<T, R> rab = ra;
     if (rab.xm2) rab.xm2 += (size_t)b0 * rab.ldx;
     rc = dispatch_sticks_fwd<T, R>(B.n3, g, st, nbb, wz, S, PrecF<R>::kin(c), inb, ld_in, outb,
                                    ld_out, ngw, rab);
+    if (rc < 0)
+      rc = any_sticks_fwd<T, R>(B, g, st, nbb, wz, S, PrecF<R>::kin(c), inb, ld_in, outb, ld_out,
+                                ngw, rab);
     timing_end(c, kFamSticksFwd, e2);
     c->kernel_launches++;
-    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: length not compiled") : rc;
+    if (rc) return rc < 0 ? fail(PSPW_ERR_NOT_IMPL, "register-FFT path: no kernel for this length") : rc;
   }
   timing_end(c, kFamLocal, ev);
   PSPW_CUDA(cudaGetLastError());

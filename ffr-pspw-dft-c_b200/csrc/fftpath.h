@@ -29,8 +29,17 @@ struct FastGeo {
   const unsigned short *sg_off = nullptr;
 };
 
-// True when (n1, n2, n3) has compiled stick and plane kernels.
-bool fast_supported(int n1, int n2, int n3);
+// Factors of a length for the register FFT (fftpath_f32.cu).
+Split split_for(int n);
+
+// Sets the basis's splits and which paths its grid takes (n1, n2, n3 and nxa
+// set).
+void set_fft_paths(Basis *B);
+
+template <typename R>
+inline bool fast_path(const Basis &B) {
+  return sizeof(R) == 8 ? B.fast64 : B.fast32;
+}
 
 // The Chebyshev recurrence applied by the last local pass:
 // out = ca * (H_loc in) + cb * in + cg * xm2 when `on`.
@@ -41,6 +50,22 @@ struct RecArg {
   const T *xm2 = nullptr;
   int ldx = 0;
 };
+
+// Stick and plane kernels with run-time lengths (fftany.cuh), for the shapes
+// without compiled ones.
+template <typename T, typename R>
+int any_plane(const Basis &B, const FastGeo &g, cudaStream_t st, int nbb, const T *wx,
+              const T *wy, const R *vperm, T *S);
+template <typename T>
+int any_plane_rho(const Basis &B, const FastGeo &g, cudaStream_t st, int ngroups, const T *wx,
+                  const T *wy, const T *S, int nbb, int bpg, const double *wband, double *part);
+template <typename T>
+int any_sticks_inv(const Basis &B, const FastGeo &g, cudaStream_t st, int nbb, const T *wz,
+                   const T *in, int ld, int ngw, T *S);
+template <typename T, typename R>
+int any_sticks_fwd(const Basis &B, const FastGeo &g, cudaStream_t st, int nbb, const T *wz,
+                   const T *S, const R *kin, const T *in, int ld, T *out, int ldo, int ngw,
+                   const RecArg<T, R> &ra);
 
 // Local part (kinetic + V_eff sandwich) of H*psi for nb bands:
 // out = kin*in + FFT^-1 sandwich (or the recurrence of ra), on the cell

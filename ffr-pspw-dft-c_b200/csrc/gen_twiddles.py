@@ -28,7 +28,7 @@ def cos_sin(m, n):
         c, s = -s, c
     return c + 0.0, s + 0.0
 
-SIZES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16]
+SIZES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16]
 
 
 def main():

@@ -1,8 +1,11 @@
 // Block H*psi on the device (the work of ApplyHam_block.cpp:5-172).
 //
 // Local part: the scatter -> inverse 3D FFT -> V_eff -> forward 3D FFT ->
-// gather chain of ApplyHam_block.cpp:33-61, done as five passes that only
-// touch the part of the grid the wavefunction sphere can reach:
+// gather chain of ApplyHam_block.cpp:33-61.  Grids whose lengths split into
+// two register factors and whose plane fits in shared memory take the fused
+// kernels of fftpath.cuh (compiled lengths) or fftany.cuh (any others); the
+// rest take five passes here that only touch the part of the grid the
+// wavefunction sphere can reach:
 //   1 sticks_inv   gather psi(G) of each stick (an (i1,i2) column holding
 //                  sphere G's) into shared memory, inverse FFT along z,
 //                  write the stick buffer S[band][z][stick]
@@ -876,7 +879,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
   // ---- local part, in batches of bands
   Geo geo{B.n1, B.n2, B.n3, B.ncol, B.nxa, B.ngw, B.d_col_start, B.d_sg_ig, B.d_sg_z,
           B.d_sg_col, B.d_col_of_xy, B.d_xa_list, B.d_xa_of_x};
-  if (B.fast) {
+  if (fast_path<R>(B)) {
     const FastGeo fg{B.ncol,    B.nxa,       B.d_col_start, B.d_sg_ig,
                      B.d_sg_z,  B.d_sg_col,  B.d_xa_list,   B.d_col_x,
                      B.d_col_y, B.d_xa_of_x, c->stick.active, B.d_sg_off};
@@ -952,7 +955,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
   // forward stick pass has applied the recurrence to the local part already
   // (out = a H_loc in + b in + g xm2), so the back-projection only adds
   // a * beta W beta^H in.
-  const bool pre = B.fast;
+  const bool pre = fast_path<R>(B);
   if (nproj > 0) {
     if (overlap) PSPW_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
     timing_begin(c, kFamNonlocal, &ev);

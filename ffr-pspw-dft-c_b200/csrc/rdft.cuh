@@ -1,8 +1,8 @@
 // Small DFTs held entirely in registers, with compile-time size and sign.
 //
 // RDft<N, S>::run(v) replaces v[k] by sum_n v[n] exp(S*2*pi*i*n*k/N).  Sizes
-// 2, 3, 4, 5 have closed-form butterflies, 7 a direct sum with constant
-// twiddles; every other size N = A*B is split by Cooley-Tukey with input
+// 2, 3, 4, 5 have closed-form butterflies, 7, 11 and 13 a sum over symmetric
+// pairs; every other size N = A*B is split by Cooley-Tukey with input
 // index n = b + B*a and output index k = ka + A*kb:
 //   X[ka + A*kb] = sum_b w_B^{b*kb} w_N^{b*ka} sum_a w_A^{a*ka} x[b + B*a].
 // All loops unroll and every twiddle is a compile-time constant
@@ -131,21 +131,45 @@ struct RDft<5, S> {
   }
 };
 
-template <int S>
-struct RDft<7, S> {
+// Odd primes up to 13, over the pairs a_j = v[j] + v[P-j], b_j = v[j] - v[P-j]:
+//   X[k], X[P-k] = v[0] + sum_j a_j cos(2 pi jk/P)  +-  S i sum_j b_j sin(2 pi jk/P),
+// (P-1)^2 real multiply-adds instead of the direct sum's 4 (P-1)^2.
+template <int P, int S>
+struct RDftOdd {
   template <typename T>
   __device__ __forceinline__ static void run(T *v) {
-    T o[7];
+    using R = decltype(T::x);
+    constexpr int H = (P - 1) / 2;
+    T a[H], b[H];
 #pragma unroll
-    for (int k = 0; k < 7; k++) {
-      T acc = v[0];
-#pragma unroll
-      for (int n = 1; n < 7; n++) acc = acc + rmul(v[n], tw_cos(7, n * k), S * tw_sin(7, n * k));
-      o[k] = acc;
+    for (int j = 0; j < H; j++) {
+      a[j] = v[1 + j] + v[P - 1 - j];
+      b[j] = v[1 + j] - v[P - 1 - j];
     }
+    const T x0 = v[0];
 #pragma unroll
-    for (int k = 0; k < 7; k++) v[k] = o[k];
+    for (int j = 0; j < H; j++) v[0] = v[0] + a[j];
+#pragma unroll
+    for (int k = 1; k <= H; k++) {
+      T m = x0, q = czero<T>();
+#pragma unroll
+      for (int j = 1; j <= H; j++) {
+        const R c = (R)tw_cos(P, j * k), s = (R)tw_sin(P, j * k);
+        m = mk<T>(m.x + c * a[j - 1].x, m.y + c * a[j - 1].y);
+        q = mk<T>(q.x + s * b[j - 1].x, q.y + s * b[j - 1].y);
+      }
+      q = mul_i<S>(q);
+      v[k] = m + q;
+      v[P - k] = m - q;
+    }
   }
 };
+
+template <int S>
+struct RDft<7, S> : RDftOdd<7, S> {};
+template <int S>
+struct RDft<11, S> : RDftOdd<11, S> {};
+template <int S>
+struct RDft<13, S> : RDftOdd<13, S> {};
 
 }  // namespace pspw
