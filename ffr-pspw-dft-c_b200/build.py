@@ -35,7 +35,7 @@ CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fvisibility=hid
 # libpspw_gpu.so
 GPU_SOURCES = ["basis.cpp", "cell.cu", "hpsi.cu", "fftpath_f32.cu", "fftpath_f64.cu", "fftany_plane_f32.cu",
                "fftany_plane_f64.cu", "fftany_sticks_f32.cu", "fftany_sticks_f64.cu", "capi.cu",
-               "noalloc.cu", "gemm.cu", "heev.cu", "dense.cu", "solvers.cu", "capi_solvers.cu", "nl_tc.cu",
+               "noalloc.cu", "gemm.cu", "fold.cu", "heev.cu", "dense.cu", "solvers.cu", "capi_solvers.cu", "nl_tc.cu",
                "scf.cu", "scf_driver.cu", "input.cpp", "geom.cu", "serve.cpp", "batch.cu"]
 GPU_LIBS = ["-lcusolver", "-lcublas", "-lcudart"]
 # libpspw_dropin.so (links libpspw_gpu.so)

@@ -20,6 +20,7 @@
 #include "nl_tc.h"
 #include "fft2.cuh"
 #include "fftpath.h"
+#include "fold.h"
 
 namespace pspw {
 
@@ -245,7 +246,8 @@ int pspw_cell_destroy(pspw_cell *c) {
                   c->d_vperm32, c->proj.d_etp, c->proj.d_etb, B.d_wgrid, c->proj.d_beta64,
                   c->stick.sg_ig, c->stick.kin64, c->stick.kin32, c->stick.eigr64,
                   c->stick.eigr32, c->stick.pkga64, c->stick.pkga32, c->stick.etp,
-                  c->stick.etb, c->stick.beta64};
+                  c->stick.etb, c->stick.beta64, c->proj.fold_mem,
+                  c->proj.fold.d_b64, c->stick.fold.d_b64};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int i = 0; i < 3; i++) {
@@ -524,6 +526,8 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
       cudaHostGetDevicePointer((void **)&c->d_err, c->h_err, 0) != cudaSuccess)
     return bail(fail(PSPW_ERR_OOM, "cell_create: error word"));
   *c->h_err = 0;
+  if ((rc = pspw::fold_prepare(c, gi1.data(), gi2.data(), gi3.data(), order.data())))
+    return bail(rc);
   if ((rc = pspw::nl_tc_prepare(c))) return bail(rc);
   *out = c;
   return PSPW_OK;
@@ -592,6 +596,7 @@ int swap_stick_order(pspw_cell *c) {
   std::swap(P.d_etp, S.etp);
   std::swap(P.d_etb, S.etb);
   std::swap(P.d_beta64, S.beta64);
+  std::swap(P.fold, S.fold);
   S.active = !S.active;
   return PSPW_OK;
 }

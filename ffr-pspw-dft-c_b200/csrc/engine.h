@@ -67,6 +67,17 @@ struct Basis {
   int *d_pinv[3] = {nullptr, nullptr, nullptr};
 };
 
+// Pairs (+G, -G) of the sphere, when every projector is even or odd under
+// G -> -G and EIGR(-G) = conj(EIGR(G)) to the last bit (fold.cu): the
+// projector products then run over pairs with real matrices.  Each order of
+// G (the cell's and the stick lists') has its pair table and matrices.
+struct Fold {
+  bool ok = false;
+  int groups = 0;           // groups of 8 pairs (the last padded)
+  int2 *d_pair = nullptr;   // [8 * groups] G indices of the pair; y < 0: G = 0, x < 0: padding
+  double *d_b64 = nullptr;  // [16 * groups x nproj] column-major, built on first use
+};
+
 // KB projectors beta_p(G) = EIGR(G, atom_p) * PKG_A(lm_p, G, species_p).
 struct Projectors {
   int nat = 0, nsp = 0, nproj = 0;
@@ -78,6 +89,9 @@ struct Projectors {
   // column-major matrix, built on the first FP64 projector call (the DMMA
   // GEMMs of gemm.cu use it as an operand)
   double2 *d_beta64 = nullptr;
+  Fold fold;
+  void *fold_mem = nullptr;        // holds the pair tables of both orders and d_odd
+  unsigned char *d_odd = nullptr;  // [nproj] projector p is odd under G -> -G
   int *d_patom = nullptr;    // [nproj] atom (species-major global index)
   int *d_psp = nullptr;      // [nproj] species
   int *d_plm = nullptr;      // [nproj] lm (0..3)
@@ -210,6 +224,7 @@ struct pspw_cell {
     float *pkga32 = nullptr;
     float *etp = nullptr, *etb = nullptr;
     double2 *beta64 = nullptr;
+    pspw::Fold fold;
   } stick;
   // Error word the kernels raise when a bounded wait gives up (pinned,
   // mapped host memory: d_err is its device alias).  Read after every

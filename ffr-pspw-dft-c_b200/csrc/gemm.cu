@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "dense.h"
+#include "dmma.cuh"
 #include "engine.h"
 #include "gemm.h"
 #include "tc.cuh"
@@ -298,17 +299,6 @@ struct Dm {
   static constexpr size_t SMEM = sizeof(double2) * STAGE * STAGES;
   static constexpr int MIN_BLOCKS = 16 / (WM * WN);  // 2, 4 or 8 blocks of registers per SM
 };
-
-// d(16 x 8) += a(16 x 4) b(4 x 8), FP64: lane (g = lane / 4, t = lane % 4)
-// holds a = A[g][t], A[g+8][t]; b = B[t][g]; d = D[g][2t], D[g][2t+1],
-// D[g+8][2t], D[g+8][2t+1]
-__device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, double b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
-      "{%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
 
 // part or C over the block's K slice [blockIdx.z * kchunk, +kchunk)
 template <bool CONJ_A, int WM, int WN>

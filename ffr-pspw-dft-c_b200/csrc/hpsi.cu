@@ -30,9 +30,10 @@
 // reduced in a fixed order, so results are deterministic) and
 // back-projection, whose epilogue also applies out = a*(H psi) + b*psi + g*x,
 // the update of the Chebyshev three-term recurrence (chebyfilt.cpp:36-59).
-// FP64: beta stored once per cell (NGW x nproj) and both products on the
-// engine's FP64 tensor-core GEMM (gemm.cu, DMMA), the recurrence as a
-// separate pass; the allocation-free entry point keeps the SIMT kernels.
+// FP64: products over pairs (+G, -G) with a real projector matrix on the FP64
+// tensor-core instruction (fold.cu); without that symmetry, or over fewer G,
+// beta stored once per cell (NGW x nproj) and both products on the complex
+// GEMM (gemm.cu).  The allocation-free entry point keeps the SIMT kernels.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +44,7 @@
 #include "engine.h"
 #include "fft.cuh"
 #include "fftpath.h"
+#include "fold.h"
 #include "gemm.h"
 #include "nl_tc.h"
 
@@ -773,17 +775,23 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
   // FP32 with one species: projector GEMMs on the tensor cores
   bool use_tc = false;
   if constexpr (sizeof(R) == 4) use_tc = nproj > 0 && nl_tc_usable(c);
+  const bool fold = sizeof(R) == 8 && nproj > 0 && !plan && fold_usable(c, ngw);
   float *tc_part = nullptr, *tc_wt = nullptr;
   int tc_split = 0;
   // The projection reads psi only: it runs on the cell's second stream,
   // concurrently with the local part, and the back-projection waits for it
   // (unless the cell's overlap mode is PSPW_OVERLAP_OFF; on Si64 the
-  // concurrent form is 6 % faster in FP32 and 8 % in FP64).  Callers with a
-  // scratch plan, i.e. the allocation-free entry point, keep one stream.
+  // concurrent form is 6 % faster in FP32 and 8 % in FP64).  In the automatic
+  // mode small products (below 4 M elements of beta x bands) stay on the cell
+  // stream: such a call is bound by its launches, and the fork and join are
+  // four more driver calls.  Callers with a scratch plan, i.e. the
+  // allocation-free entry point, keep one stream.
   // c->stream is switched for the projection's launches and switched back
   // on every exit from this block.
   const cudaStream_t main_st = c->stream;
-  const bool overlap = c->nl_overlap != PSPW_OVERLAP_OFF && nproj > 0 && !plan &&
+  const bool worth = c->nl_overlap == PSPW_OVERLAP_ON ||
+                     (double)nproj * ngw * nb >= 4.0 * (1 << 20);
+  const bool overlap = c->nl_overlap != PSPW_OVERLAP_OFF && worth && nproj > 0 && !plan &&
                        c->stream2 != nullptr;
   struct StreamSwitch {
     pspw_cell *c;
@@ -809,7 +817,10 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
       part = static_cast<T *>(plan->part);
       wp = static_cast<T *>(plan->wp);
     } else {
-      if (!use_tc) {
+      if (fold) {
+        int rc = ws_reserve(c, 3, sizeof(T) * (size_t)nb * nproj, (void **)&wp);
+        if (rc) return rc;
+      } else if (!use_tc) {
         int rc = ws_reserve(c, 2, sizeof(T) * (size_t)nsplit * nb * nproj, (void **)&part);
         if (rc) return rc;
         rc = ws_reserve(c, 3, sizeof(T) * (size_t)nb * nproj, (void **)&wp);
@@ -819,8 +830,18 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
     timing_begin(c, kFamNonlocal, &ev);
     bool done = false;
     if constexpr (sizeof(R) == 8) {
-      // FP64 without a scratch plan: beta materialised once, complex GEMMs
-      if (!plan) {
+      // FP64 without a scratch plan: products over pairs (+G, -G) where the
+      // projectors have the symmetry, else beta materialised once and complex
+      // GEMMs
+      if (!plan && fold) {
+        cudaEvent_t e;
+        timing_begin(c, kFamProj, &e);
+        const int rc = fold_project64(c, reinterpret_cast<const double2 *>(in), ld_in, nb,
+                                      reinterpret_cast<double2 *>(wp), false);
+        if (rc) return rc;
+        timing_end(c, kFamProj, e);
+        done = true;
+      } else if (!plan) {
         int rc = ensure_beta64(c, pa);
         if (rc) return rc;
         cudaEvent_t e;
@@ -975,8 +996,12 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
         if (!plan) {
           cudaEvent_t e;
           timing_begin(c, kFamBackproj, &e);
-          int rc = backproject_beta64(c, reinterpret_cast<const double2 *>(wp), ngw, nb,
-                                      reinterpret_cast<double2 *>(out), ld_out, pre ? a : 1.0);
+          int rc = fold ? fold_backproject64(c, reinterpret_cast<const double2 *>(wp), nb,
+                                             reinterpret_cast<double2 *>(out), ld_out,
+                                             pre ? a : 1.0)
+                        : backproject_beta64(c, reinterpret_cast<const double2 *>(wp), ngw, nb,
+                                             reinterpret_cast<double2 *>(out), ld_out,
+                                             pre ? a : 1.0);
           if (rc) return rc;
           if (!pre && (a != 1.0 || b != 0.0 || g != 0.0)) {
             k_axpby3<R><<<4 * 148, 256, 0, st>>>(ngw, nb, out, ld_out, in, ld_in, xm2, ld_xm2,
@@ -1013,6 +1038,7 @@ int project_fp64(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, doub
   using R = double;
   const int nproj = c->proj.nproj;
   if (nproj <= 0 || nb <= 0) return PSPW_OK;
+  if (fold_usable(c, ngw)) return fold_project64(c, psi, ld, nb, P, true);
   ProjArg pa;
   pa.eigr = Prec<R>::eigr(c);
   pa.pkga = Prec<R>::pkga(c);

@@ -114,16 +114,18 @@ int pspw_cell_set_band_batch(pspw_cell *cell, int nbatch);
  * most 4 projectors per atom (one projection and one back-projection per
  * such species), else the SIMT kernels; TENSOR_CORE on a cell outside that
  * range is PSPW_ERR_NOT_IMPL.  The FP64 path does not depend on it: it stores the
- * projectors once per cell and runs both products on the FP64 tensor-core
- * GEMM (the allocation-free entry point keeps SIMT kernels). */
+ * projectors once per cell (as a real matrix over pairs of G and -G where they
+ * have that symmetry) and runs both products on the FP64 tensor-core
+ * instruction (the allocation-free entry point keeps SIMT kernels). */
 #define PSPW_NL_AUTO 0
 #define PSPW_NL_SIMT 1
 #define PSPW_NL_TENSOR_CORE 2
 int pspw_cell_set_nl_path(pspw_cell *cell, int path);
 
 /* Whether the projection of H*psi runs on the cell's second stream,
- * concurrently with the FFT passes (AUTO, ON), or after them on the cell
- * stream (OFF); no reference counterpart.  Results do not depend on it (the
+ * concurrently with the FFT passes (ON), or on the cell stream (OFF); AUTO
+ * takes the second stream where the products are large enough to gain from
+ * it; no reference counterpart.  Results do not depend on it (the
  * same kernels run in the same order of arithmetic).  The allocation-free
  * entry point always keeps one stream. */
 #define PSPW_OVERLAP_AUTO 0
