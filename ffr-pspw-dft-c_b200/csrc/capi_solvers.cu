@@ -44,32 +44,53 @@ int sync(pspw_cell *c) {
   return device_status(c);
 }
 
-// ss[j] = sum_{i<m} |c|^2, sk[j] = sum_{i<m} xkg[i] |c|^2 (EvalRhoPsi.cpp:117-126)
-__global__ void k_charge_sums(const double2 *__restrict__ X, int ld, int m,
-                              const double *__restrict__ xkg, double *ss, double *sk) {
-  __shared__ double r1[256], r2[256];
+// ss[j] = sum_{i<m} |c|^2, sk[j] = sum_{i<m} xkg[i] |c|^2 (EvalRhoPsi.cpp:117-126).
+// One block of 1024 threads per band, four loads in flight per thread (a
+// band per SM: 256 threads with one load each read 54 MB in 53 us).
+__global__ void __launch_bounds__(1024)
+    k_charge_sums(const double2 *__restrict__ X, int ld, int m, const double *__restrict__ xkg,
+                  double *ss, double *sk) {
+  __shared__ double2 red[32];
   const int j = blockIdx.x;
   const double2 *col = X + (size_t)j * ld;
-  double a = 0.0, b = 0.0;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    const double2 v = col[i];
-    const double q = v.x * v.x + v.y * v.y;
-    a += q;
-    b += xkg[i] * q;
-  }
-  r1[threadIdx.x] = a;
-  r2[threadIdx.x] = b;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      r1[threadIdx.x] += r1[threadIdx.x + w];
-      r2[threadIdx.x] += r2[threadIdx.x + w];
+  constexpr int U = 4;
+  double a[U] = {0.0}, b[U] = {0.0};
+  for (int i0 = threadIdx.x; i0 < m; i0 += U * 1024) {
+    double2 v[U];
+    double w[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * 1024;
+      v[u] = i < m ? col[i] : make_double2(0.0, 0.0);
+      w[u] = i < m ? xkg[i] : 0.0;
     }
-    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const double q = v[u].x * v[u].x + v[u].y * v[u].y;
+      a[u] += q;
+      b[u] += w[u] * q;
+    }
   }
-  if (threadIdx.x == 0) {
-    ss[j] = r1[0];
-    sk[j] = r2[0];
+  double sa = (a[0] + a[1]) + (a[2] + a[3]), sb = (b[0] + b[1]) + (b[2] + b[3]);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_down_sync(0xffffffffu, sa, o);
+    sb += __shfl_down_sync(0xffffffffu, sb, o);
+  }
+  if (lane == 0) red[warp] = make_double2(sa, sb);
+  __syncthreads();
+  if (warp != 0) return;
+  sa = red[lane].x;
+  sb = red[lane].y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_down_sync(0xffffffffu, sa, o);
+    sb += __shfl_down_sync(0xffffffffu, sb, o);
+  }
+  if (lane == 0) {
+    ss[j] = sa;
+    sk[j] = sb;
   }
 }
 
@@ -100,7 +121,7 @@ int eval_rho_psi_dev(pspw_cell *c, const double2 *dX, int ld, int ngw, int nx, c
   std::vector<double> wband(nx);
   for (int i = 0; i < nx; i++) wband[i] = (wkpt * focc[i]) / omega;
   PSPW_CUDA(cudaMemcpyAsync(dw, wband.data(), sizeof(double) * nx, cudaMemcpyHostToDevice, c->stream));
-  k_charge_sums<<<nx, 256, 0, c->stream>>>(dX, ld, m, B.d_xkg64, dsum, dsum + nx);
+  k_charge_sums<<<nx, 1024, 0, c->stream>>>(dX, ld, m, B.d_xkg64, dsum, dsum + nx);
   c->kernel_launches++;
   if (B.fast_rho) {
     const FastGeo g{B.ncol,    B.nxa,       B.d_col_start, B.d_sg_ig,

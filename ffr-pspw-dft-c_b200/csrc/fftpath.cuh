@@ -169,17 +169,25 @@ constexpr size_t plane_smem() {
   return sizeof(T) * ((size_t)NY * PlaneCfg<NX, NY>::LS + NX + NY) + sizeof(int) * NX;
 }
 
+// FP64 planes of 256 threads whose shared memory leaves room for three blocks
+// per SM are held to the registers of three (64 x 64: 88 -> 80)
+template <int NX, int NY, typename T>
+constexpr int plane_min_blocks() {
+  return sizeof(T) == 16 && PlaneCfg<NX, NY>::NT == 256 &&
+                 3 * (plane_smem<NX, NY, T>() + 1024) <= 228 * 1024
+             ? 3
+             : 1;
+}
+
 // One z-plane of one band.  The y transforms and the stick scatter/gather
 // work on the compact view [y][xa] (active x only, odd row stride la), the x
 // transforms on full rows [y][x] (stride LS); the two x steps at the ends of
 // the x sandwich convert between the views (x_inv_expand / x_fwd_compact).
 // Only the compact view needs clearing.
 template <int NX, int NY, typename T, typename R>
-__global__ void __launch_bounds__(PlaneCfg<NX, NY>::NT) k_plane(FastGeo g, int n3,
-                                                                const T *__restrict__ wx_g,
-                                                                const T *__restrict__ wy_g,
-                                                                const R *__restrict__ vperm,
-                                                                T *__restrict__ S) {
+__global__ void __launch_bounds__(PlaneCfg<NX, NY>::NT, plane_min_blocks<NX, NY, T>())
+    k_plane(FastGeo g, int n3, const T *__restrict__ wx_g, const T *__restrict__ wy_g,
+            const R *__restrict__ vperm, T *__restrict__ S) {
   constexpr int LS = PlaneCfg<NX, NY>::LS, NT = PlaneCfg<NX, NY>::NT;
   constexpr int AX = nsplit_for(NX).n1, BX = nsplit_for(NX).n2;
   constexpr int AY = nsplit_for(NY).n1, BY = nsplit_for(NY).n2;
@@ -419,10 +427,30 @@ int rho_fast(pspw_cell *c, const FastGeo &g, const cx<R> *psi, int ld, int ngw_s
   const Basis &B = c->basis;
   cudaStream_t st = c->stream;
   const size_t s_band = (size_t)B.n3 * B.ncol;
+  // stick buffers of about 96 MB (they stay in L2), batches of equal size
   int nbatch = c->band_batch;
-  if (nbatch <= 0) nbatch = (int)std::max<size_t>(1, (48u << 20) / (s_band * sizeof(T)));
+  if (nbatch <= 0) {
+    const int cap = (int)std::max<size_t>(1, (96u << 20) / (s_band * sizeof(T)));
+    const int nbatches = (nb + cap - 1) / cap;
+    nbatch = (nb + nbatches - 1) / nbatches;
+  }
   nbatch = std::min(nbatch, nb);
-  const int ngroups = std::max(1, std::min(nbatch, (2 * 148 + B.n3 - 1) / B.n3));
+  // Band groups per z-plane: a block takes one plane of one group, and the
+  // time goes as (waves of resident blocks) x (bands per group).  Si64, 142
+  // bands, 296 resident blocks: 9 groups, two full waves of 16 bands; 5
+  // groups of 10 bands per batch of 49 left the second wave of each of three
+  // batches nearly empty (414 us of plane kernels).
+  const size_t block_smem = sizeof(T) * (size_t)B.n2 * (B.n1 + 1) + sizeof(double) * (size_t)B.n1 * B.n2;
+  const int resident = 148 * std::max<int>(1, std::min<size_t>(2, (228 * 1024) / (block_smem + 4096)));
+  int ngroups = 1;
+  long best = 1L << 60;
+  for (int n = 1; n <= std::min(nbatch, 32); n++) {
+    const long t = (long)((B.n3 * n + resident - 1) / resident) * ((nbatch + n - 1) / n);
+    if (t < best) {
+      best = t;
+      ngroups = n;
+    }
+  }
   T *S = nullptr;
   double *part = nullptr;
   int rc;
