@@ -247,7 +247,7 @@ int pspw_cell_destroy(pspw_cell *c) {
                   c->stick.sg_ig, c->stick.kin64, c->stick.kin32, c->stick.eigr64,
                   c->stick.eigr32, c->stick.pkga64, c->stick.pkga32, c->stick.etp,
                   c->stick.etb, c->stick.beta64, c->proj.fold_mem,
-                  c->proj.fold.d_b64, c->stick.fold.d_b64};
+                  c->proj.fold.d_b64, c->stick.fold.d_b64, c->proj.fold.etp, c->stick.fold.etp};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int i = 0; i < 3; i++) {
@@ -583,7 +583,8 @@ int swap_stick_order(pspw_cell *c) {
         (rc = gather_copy(c, P.d_pkga64, P.nproj > 0 ? P.nsp : 0, 4, &S.pkga64)) ||
         (rc = gather_copy(c, P.d_pkga32, P.nproj > 0 ? P.nsp : 0, 4, &S.pkga32)))
       return rc;
-    if (P.d_etp && S.eigr32 && (rc = nl_tc_build_tiles(c, S.eigr32, &S.etp, &S.etb))) return rc;
+    // (with the pair symmetry the filter's products run over pairs only)
+    if (!P.fold.ok && P.d_etp && S.eigr32 && (rc = nl_tc_build_tiles(c, S.eigr32, &S.etp, &S.etb))) return rc;
     S.built = true;
   }
   std::swap(B.d_sg_ig, S.sg_ig);

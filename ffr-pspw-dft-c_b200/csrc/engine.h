@@ -76,6 +76,9 @@ struct Fold {
   int groups = 0;           // groups of 8 pairs (the last padded)
   int2 *d_pair = nullptr;   // [8 * groups] G indices of the pair; y < 0: G = 0, x < 0: padding
   double *d_b64 = nullptr;  // [16 * groups x nproj] column-major, built on first use
+  // FP32 operand tiles of the tensor-core GEMMs over pairs (nl_tc.cu), built on
+  // first use; etb points into etp's allocation
+  float *etp = nullptr, *etb = nullptr;
 };
 
 // KB projectors beta_p(G) = EIGR(G, atom_p) * PKG_A(lm_p, G, species_p).
@@ -103,6 +106,7 @@ struct Projectors {
   float *d_etb = nullptr;  // back-projection: per (128 G, 8 atoms), [128 x 16] hi then lo
   // (both hold one block of tiles per species with projectors, species in order)
   int tc_npad = 0;         // atoms padded to a multiple of 16 (largest species)
+  std::vector<unsigned> sp_odd;   // per species: bit lm set when the form factor is odd (host)
   std::vector<int> sp_na, sp_lm;  // per species: atoms, projectors per atom (host)
 };
 

@@ -623,6 +623,10 @@ int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, c
       for (int lm = 0; lm < P.sp_lm[s]; lm++)
         if (P.sp_na[s] > 0)
           ok = ok && (flags[1 + 2 * (4 * s + lm)] || flags[2 + 2 * (4 * s + lm)]);
+    P.sp_odd.assign(P.nsp, 0u);
+    for (int s = 0; s < P.nsp; s++)
+      for (int lm = 0; lm < 4; lm++)
+        if (!flags[1 + 2 * (4 * s + lm)]) P.sp_odd[s] |= 1u << lm;
     for (int s = 0; s < P.nsp; s++)
       for (int a = 0; a < P.sp_na[s]; a++)
         for (int lm = 0; lm < P.sp_lm[s]; lm++) odd.push_back(!flags[1 + 2 * (4 * s + lm)]);

@@ -775,7 +775,8 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
   // FP32 with one species: projector GEMMs on the tensor cores
   bool use_tc = false;
   if constexpr (sizeof(R) == 4) use_tc = nproj > 0 && nl_tc_usable(c);
-  const bool fold = sizeof(R) == 8 && nproj > 0 && !plan && fold_usable(c, ngw);
+  // products over pairs (+G, -G) where the projectors have that symmetry
+  const bool fold = (sizeof(R) == 8 || use_tc) && nproj > 0 && !plan && fold_usable(c, ngw);
   float *tc_part = nullptr, *tc_wt = nullptr;
   int tc_split = 0;
   // The projection reads psi only: it runs on the cell's second stream,
@@ -817,7 +818,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
       part = static_cast<T *>(plan->part);
       wp = static_cast<T *>(plan->wp);
     } else {
-      if (fold) {
+      if (fold && !use_tc) {
         int rc = ws_reserve(c, 3, sizeof(T) * (size_t)nb * nproj, (void **)&wp);
         if (rc) return rc;
       } else if (!use_tc) {
@@ -864,13 +865,14 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
         tc_wt = static_cast<float *>(plan->wt);
         tc_split = plan->max_split;
       } else {
-        const int rc = nl_tc_reserve(c, ngw, nb, &tc_part, &tc_split, &tc_wt);
+        int rc = fold ? nl_tc_pair_tiles(c) : PSPW_OK;
         if (rc) return rc;
+        if ((rc = nl_tc_reserve(c, ngw, nb, &tc_part, &tc_split, &tc_wt, fold))) return rc;
       }
       cudaEvent_t e;
       timing_begin(c, kFamProj, &e);
       const int rc = nl_tc_project(c, reinterpret_cast<const float2 *>(in), ld_in, ngw, nb,
-                                   tc_part, tc_split, tc_wt);
+                                   tc_part, tc_split, tc_wt, fold);
       timing_end(c, kFamProj, e);
       if (rc) return rc;
     } else {
@@ -986,7 +988,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
       const int rc = nl_tc_backproject(
           c, tc_wt, ngw, nb, reinterpret_cast<float2 *>(out), ld_out,
           reinterpret_cast<const float2 *>(in), ld_in, reinterpret_cast<const float2 *>(xm2),
-          ld_xm2, (float)a, pre ? 0.f : (float)b, pre ? 0.f : (float)g, pre);
+          ld_xm2, (float)a, pre ? 0.f : (float)b, pre ? 0.f : (float)g, pre, fold);
       timing_end(c, kFamBackproj, e);
       if (rc) return rc;
     } else {

@@ -21,6 +21,17 @@
 //   K = 2*atoms; the epilogue contracts lm with PKG and applies the
 //   Chebyshev update out = a (H psi) + b psi + g x.
 //
+// Where the projectors have the symmetry of fold.cu (every Gamma-point cell
+// built from atoms), both GEMMs run over pairs (+G, -G) instead of G, at half
+// the operations and half the operand bytes.  With u, d = psi(G) +- psi(-G)
+// and (a, b) = (u, d) for even and (d, u) for odd form factors:
+//   projection: the same B' (E at +G) against
+//     A'[(b,lm,re)][(pair,*)] = PKG (Re a,  Im b)
+//     A'[(b,lm,im)][(pair,*)] = PKG (Im a, -Re b)
+//   back-projection: two accumulators per tile of 128 pairs, T1 with A' = Re E
+//     and T2 with A' = Im E, both against W as it is (K = atoms), and
+//     NL(+-G) = sum_lm PKG(+-G) (T1 +- i T2) in the epilogue.
+//
 // Operands that do not depend on psi (both EIGR operands) are split into
 // TF32 hi/lo tiles once per cell, in the K-major no-swizzle layout of tc.cuh,
 // and reach shared memory as single bulk copies.  The psi operand of the
@@ -154,16 +165,23 @@ __device__ __forceinline__ void drain_bulk(Sync &sy, int issued, int nt) {
 __host__ __device__ constexpr int proj_slots(int npad) { return tmem_cols(npad) <= 64 ? 3 : 2; }
 constexpr int kStepG = 16;  // G per projection step
 
-template <int L>
+// FOLD: ngw counts pairs (table `pair`), a raw row holds psi at +G and at -G,
+// and bit lm of `odd` marks the odd form factors.
+__host__ __device__ constexpr int raw_row(bool fold) { return (fold ? 2 : 1) * (kStepG + 1); }
+
+template <int L, bool FOLD>
 __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict__ psi, int ld,
                                                       int ngw, int nb,
                                                       const float *__restrict__ etp,
                                                       const float *__restrict__ pkga, int nat,
                                                       int npad, int ksplit_g,
-                                                      float *__restrict__ part, int *err) {
+                                                      float *__restrict__ part, int *err,
+                                                      const int2 *__restrict__ pair,
+                                                      unsigned odd) {
   constexpr int per = 2 * L;
   constexpr int nbr_max = 127 / per + 2;  // bands a 128-row tile touches
-  constexpr int prow = kStepG + 1;        // raw psi row (float2), padded
+  constexpr int prow = raw_row(FOLD);     // raw psi row (float2), padded
+  constexpr int kMinus = kStepG + 1;      // FOLD: where the -G values start
   constexpr int raw_psi = round16(nbr_max * prow * 8);
   constexpr int raw_bytes = raw_psi + kStepG * 16;
   extern __shared__ __align__(1024) unsigned char sm[];
@@ -190,6 +208,7 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
     const bool mv = m < Mtot;
     const int bl = mv ? m / per - bfirst : 0;
     const int lm = (m % per) >> 1, p = m & 1;
+    const bool is_odd = FOLD && ((odd >> lm) & 1);
     for (int k = 0; k < nsteps; k++) {
       const int rs = k % kNR, ts = k % nts;
       if (!tc::mbar_wait_abort(&sy.rfull[rs], (k / kNR) & 1, &sy.abort)) break;
@@ -203,8 +222,17 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
       for (int j = 0; j < 8; j++) {
         const float2 v = rp[j];
         const float f = rk[4 * j];
-        const float x0 = p ? f * v.y : f * v.x;
-        const float x1 = p ? -f * v.x : f * v.y;
+        float x0, x1;
+        if constexpr (FOLD) {
+          const float2 q = rp[kMinus + j];
+          const float2 u = v + q, d = v - q;
+          const float2 a = is_odd ? d : u, b = is_odd ? u : d;
+          x0 = p ? f * a.y : f * a.x;
+          x1 = p ? -f * b.x : f * b.y;
+        } else {
+          x0 = p ? f * v.y : f * v.x;
+          x1 = p ? -f * v.x : f * v.y;
+        }
         tc::split_tf32(mv ? x0 : 0.f, hi[2 * j], lo[2 * j]);
         tc::split_tf32(mv ? x1 : 0.f, hi[2 * j + 1], lo[2 * j + 1]);
       }
@@ -241,24 +269,44 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
       }
     }
   } else if (warp == kRowWarps) {
-    // ---- raw producer: psi / PKG_A by all lanes
+    // ---- raw producer: psi / PKG_A by all lanes (FOLD: lane's pair of a step
+    // is read one step ahead)
+    auto pair_at = [&](int k) {
+      const int g = gb + kStepG * k + (lane & (kStepG - 1));
+      return FOLD && g < ge ? pair[g] : make_int2(-1, -1);
+    };
+    int2 next = pair_at(0);
     for (int k = 0; k < nsteps; k++) {
       const int rs = k % kNR;
+      const int2 pr = next;
+      next = pair_at(k + 1);
       if (k >= kNR && !tc::mbar_wait_abort(&sy.rempty[rs], ((k / kNR) - 1) & 1, &sy.abort))
         break;
       unsigned char *r = raw0 + rs * raw_bytes;
       float2 *rp = reinterpret_cast<float2 *>(r);
       float *rk = reinterpret_cast<float *>(r + raw_psi);
       const int g0 = gb + kStepG * k;
-      for (int e = lane; e < nbr * kStepG; e += 32) {
-        const int b = e / kStepG, j = e % kStepG, g = g0 + j;
-        const bool v = g < ge;
-        tc::cp_async8(rp + b * prow + j, psi + (size_t)(bfirst + b) * ld + (v ? g : 0), v);
-      }
-      if (lane < kStepG) {
-        const int g = g0 + lane;
-        const bool v = g < ge;
-        tc::cp_async16(rk + 4 * lane, pkga + (size_t)(v ? g : 0) * 4, v);
+      if constexpr (FOLD) {
+        const int j = lane & (kStepG - 1);
+        const bool vx = pr.x >= 0, vy = pr.y >= 0;
+        const float2 *px = psi + (size_t)bfirst * ld + (vx ? pr.x : 0);
+        const float2 *py = psi + (size_t)bfirst * ld + (vy ? pr.y : 0);
+        for (int b = lane / kStepG; b < nbr; b += 32 / kStepG) {
+          tc::cp_async8(rp + b * prow + j, px + (size_t)b * ld, vx);
+          tc::cp_async8(rp + b * prow + kMinus + j, py + (size_t)b * ld, vy);
+        }
+        if (lane < kStepG) tc::cp_async16(rk + 4 * lane, pkga + (size_t)(vx ? pr.x : 0) * 4, vx);
+      } else {
+        for (int e = lane; e < nbr * kStepG; e += 32) {
+          const int b = e / kStepG, j = e % kStepG, g = g0 + j;
+          const bool v = g < ge;
+          tc::cp_async8(rp + b * prow + j, psi + (size_t)(bfirst + b) * ld + (v ? g : 0), v);
+        }
+        if (lane < kStepG) {
+          const int g = g0 + lane;
+          const bool v = g < ge;
+          tc::cp_async16(rk + 4 * lane, pkga + (size_t)(v ? g : 0) * 4, v);
+        }
       }
       tc::cp_async_mbar_arrive_noinc(&sy.rfull[rs]);
     }
@@ -314,8 +362,10 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
 // 2 pair, 2 pair + 1) over slices q, q + 4, ..., so a warp reads whole rows
 // of part; the four partial sums are added in the order q = 0..3, so the
 // result does not depend on scheduling.
+// FOLD: tile (bt, s) holds ncolN rows x 16 atoms of W itself (rows re, im),
+// 8 atom pairs per step.
 constexpr int kWtWarps = 4;
-template <int L>
+template <int L, bool FOLD>
 __global__ void __launch_bounds__(32 * kWtWarps) k_proj_tc_wtiles(
     const float *__restrict__ part, int nsplit, int nb, int nat, const float *__restrict__ w,
     int nbt, int nsa, float *__restrict__ wt) {
@@ -345,7 +395,7 @@ __global__ void __launch_bounds__(32 * kWtWarps) k_proj_tc_wtiles(
   }
   ps[q][lane] = x;
   __syncthreads();
-  if (q != 0 || pair >= 4 * nsa) return;
+  if (q != 0 || pair >= (FOLD ? 8 : 4) * nsa) return;
 #pragma unroll
   for (int i = 1; i < kWtWarps; i++) {
     const float4 y = ps[i][lane];
@@ -357,12 +407,26 @@ __global__ void __launch_bounds__(32 * kWtWarps) k_proj_tc_wtiles(
   const float w0 = a0 < nat ? w[a0 * L + lm] : 0.f;
   const float w1 = a0 + 1 < nat ? w[(a0 + 1) * L + lm] : 0.f;
   const float2 W0 = make_float2(w0 * x.x, w0 * x.y), W1 = make_float2(w1 * x.z, w1 * x.w);
-  const int s = pair >> 2, c = pair & 3;
+  const int s = FOLD ? pair >> 3 : pair >> 2, c = FOLD ? pair & 7 : pair & 3;
   const int bt = b / nbt, bl = b % nbt;
   const int ncolN = nbt * per;
   unsigned char *hi = reinterpret_cast<unsigned char *>(wt + ((size_t)bt * nsa + s) * ncolN * 32);
   unsigned char *lo = hi + ncolN * 64;
   const int r = bl * per + 2 * lm;
+  if constexpr (FOLD) {
+    uint2 h, l;
+    tc::split_tf32(W0.x, h.x, l.x);
+    tc::split_tf32(W1.x, h.y, l.y);
+    const uint32_t o = tc::core_off<kBK>(r, 2 * c);
+    *reinterpret_cast<uint2 *>(hi + o) = h;
+    *reinterpret_cast<uint2 *>(lo + o) = l;
+    tc::split_tf32(W0.y, h.x, l.x);
+    tc::split_tf32(W1.y, h.y, l.y);
+    const uint32_t o1 = tc::core_off<kBK>(r + 1, 2 * c);
+    *reinterpret_cast<uint2 *>(hi + o1) = h;
+    *reinterpret_cast<uint2 *>(lo + o1) = l;
+    return;
+  }
   tc::st_split4(hi, lo, tc::core_off<kBK>(r, 4 * c), make_float4(W0.x, -W0.y, W1.x, -W1.y));
   tc::st_split4(hi, lo, tc::core_off<kBK>(r + 1, 4 * c), make_float4(W0.y, W0.x, W1.y, W1.x));
 }
@@ -514,6 +578,156 @@ __global__ void __launch_bounds__(kThreads) k_backproj_tc(
   close_block(sy, ncols, err);
 }
 
+// Over pairs: grid (tiles of 128 pairs, band tiles of nbt); kThreads threads.
+// etb: per (128 pairs, 16 atoms), Re E [128 x 16] hi, lo, then Im E hi, lo.
+// D: columns [0, ncolN) = T1 (Re E), the same from t2_col(ncolN) on = T2 (Im E).  Epilogue
+// thread (warp w, lane l): pair 32 (w % 4) + l, bands of half w / 4.
+__host__ __device__ constexpr int t2_col(int ncolN) { return (ncolN + 31) & ~31; }
+
+template <int L, bool PRE>
+__global__ void __launch_bounds__(kThreads) k_backpair_tc(
+    const float *__restrict__ etb, const float *__restrict__ wt, int nsa, int npair,
+    const int2 *__restrict__ pair, unsigned odd, int nb, int nbt, const float *__restrict__ pkga,
+    float2 *out, int ldo, const float2 *__restrict__ in, int ldi, const float2 *__restrict__ xm2,
+    int ldx, float ca, float cb, float cg, int *err) {
+  constexpr int per = 2 * L;
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ Sync sy;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gt = blockIdx.x, bt = blockIdx.y;
+  const int b0 = bt * nbt;
+  const int nbb = min(nbt, nb - b0);
+  const int ncolN = nbt * per;  // a multiple of 16, <= 128; nbt is even
+  const uint32_t abytes = 4 * kTileBytes128, bbytes = (uint32_t)ncolN * 128;
+  const int slot_bytes = (int)(abytes + bbytes);
+  const uint32_t ncols = tmem_cols(2 * t2_col(ncolN));
+  open_block(sy, ncols, kNTB, 1, 0);
+
+  if (warp == kRowWarps) {
+    if (lane == 0) {
+      int issued = 0;
+      for (int k = 0; k < nsa; k++) {
+        const int ts = k % kNTB;
+        if (k >= kNTB && !tc::mbar_wait_abort(&sy.empty[ts], ((k / kNTB) - 1) & 1, &sy.abort))
+          break;
+        unsigned char *slot = sm + ts * slot_bytes;
+        tc::mbar_arrive_expect_tx(&sy.bfull[ts], abytes + bbytes);
+        tc::bulk_g2s(slot, etb + ((size_t)gt * nsa + k) * (abytes / 4), abytes, &sy.bfull[ts]);
+        tc::bulk_g2s(slot + abytes, wt + ((size_t)bt * nsa + k) * (bbytes / 4), bbytes,
+                     &sy.bfull[ts]);
+        issued = k + 1;
+      }
+      drain_bulk(sy, issued, kNTB);
+    }
+  } else if (warp == kRowWarps + 1) {
+    if (lane == 0) {
+      const uint32_t idesc = tc::idesc_tf32(128, ncolN);
+      for (int k = 0; k < nsa; k++) {
+        const int ts = k % kNTB;
+        if (!tc::mbar_wait_abort(&sy.bfull[ts], (k / kNTB) & 1, &sy.abort)) break;
+        tc::fence_after_sync();
+        const uint32_t a = tc::smem_addr(sm + ts * slot_bytes);
+        const uint32_t b = a + abytes;
+        issue_step(sy.tmem, a, a + kTileBytes128, b, b + ncolN * 64, idesc, k == 0);
+        issue_step(sy.tmem + t2_col(ncolN), a + 2 * kTileBytes128, a + 3 * kTileBytes128, b,
+                   b + ncolN * 64, idesc, k == 0);
+        tc::mma_commit(&sy.empty[ts]);
+      }
+      tc::mma_commit(&sy.done);
+    }
+  } else {
+    // ---- epilogue
+    const int row = 32 * (warp & 3) + lane, half = warp >> 2;
+    const uint32_t lane_base = sy.tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const int j = gt * 128 + row;
+    const int2 pr = j < npair ? pair[j] : make_int2(-1, -1);
+    const bool vp = pr.x >= 0, vm = pr.y >= 0;
+    const int nbh = nbt / 2;
+    const int bstart = half * nbh;
+    float pk[4] = {0.f, 0.f, 0.f, 0.f};
+    if (vp) {
+      const float4 p4 = *reinterpret_cast<const float4 *>(pkga + (size_t)pr.x * 4);
+      pk[0] = p4.x;
+      pk[1] = p4.y;
+      pk[2] = p4.z;
+      pk[3] = p4.w;
+    }
+    // operands of CH bands at +G and -G at once (the first while the MMAs run)
+    constexpr int CH = PRE ? 8 : 2;
+    float2 hv[CH][2], uv[CH][2], xv[CH][2];
+    auto fetch = [&](int j0) {
+#pragma unroll
+      for (int i = 0; i < CH; i++) {
+        const int bl = bstart + j0 + i;
+        const bool on = j0 + i < nbh && bl < nbb;
+        const size_t bb = (size_t)(b0 + bl);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const int g = q ? pr.y : pr.x;
+          hv[i][q] = uv[i][q] = xv[i][q] = make_float2(0.f, 0.f);
+          if (on && g >= 0) {
+            hv[i][q] = out[bb * ldo + g];
+            if (!PRE && cb != 0.f) uv[i][q] = in[bb * ldi + g];
+            if (!PRE && cg != 0.f) xv[i][q] = xm2[bb * ldx + g];
+          }
+        }
+      }
+    };
+    fetch(0);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_abort(&sy.done, 0, &sy.abort));
+    tc::fence_after_sync();
+    if (ok) {
+      for (int j0 = 0; j0 < nbh; j0 += CH) {
+        if (j0 > 0) fetch(j0);
+#pragma unroll
+        for (int i = 0; i < CH; i++) {
+          const int jb = j0 + i;
+          if (jb >= nbh) break;  // block-uniform: the TMEM loads below are warp-collective
+          uint32_t t1[per], t2[per];
+          const uint32_t col = lane_base + (uint32_t)((bstart + jb) * per);
+          ld_band<per>(col, t1);
+          ld_band<per>(col + t2_col(ncolN), t2);
+          float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const float ar = __uint_as_float(t1[2 * l]), ai = __uint_as_float(t1[2 * l + 1]);
+            const float br = __uint_as_float(t2[2 * l]), bi = __uint_as_float(t2[2 * l + 1]);
+            const float f = pk[l], fm = (odd >> l) & 1 ? -f : f;
+            acc[0].x += f * (ar - bi);
+            acc[0].y += f * (ai + br);
+            acc[1].x += fm * (ar + bi);
+            acc[1].y += fm * (ai - br);
+          }
+          const int bl = bstart + jb;
+          if (bl >= nbb) continue;
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            if (!(q ? vm : vp)) continue;
+            const int g = q ? pr.y : pr.x;
+            const float2 hc = hv[i][q];
+            float2 r;
+            if (PRE) {
+              r = make_float2(hc.x + ca * acc[q].x, hc.y + ca * acc[q].y);
+            } else {
+              r = make_float2(ca * (hc.x + acc[q].x), ca * (hc.y + acc[q].y));
+              if (cb != 0.f) {
+                r.x += cb * uv[i][q].x;
+                r.y += cb * uv[i][q].y;
+              }
+              if (cg != 0.f) {
+                r.x += cg * xv[i][q].x;
+                r.y += cg * xv[i][q].y;
+              }
+            }
+            out[(size_t)(b0 + bl) * ldo + g] = r;
+          }
+        }
+      }
+    }
+  }
+  close_block(sy, ncols, err);
+}
+
 // ------------------------------------------------------------------ EIGR tiles
 __global__ void k_build_etp(const float2 *__restrict__ eigr, int ngw, int nat, int npad, int nst,
                             float *__restrict__ etp) {
@@ -560,6 +774,52 @@ __global__ void k_build_etb(const float2 *__restrict__ eigr, int ngw, int nat, i
   tc::st_split4(hi, hi + 8192, tc::core_off<kBK>(gg, 4 * c), make_float4(v[0], v[1], v[2], v[3]));
 }
 
+// The same operands over pairs: projection tiles per 8 pairs, E at +G;
+__global__ void k_build_etp_pairs(const float2 *__restrict__ eigr, const int2 *__restrict__ pair,
+                                  int npair, int ngw, int nat, int npad, int nst,
+                                  float *__restrict__ etp) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (idx >= (long long)nst * npad * 4) return;
+  const int c = (int)(idx & 3);
+  const int r = (int)((idx >> 2) % npad);
+  const int s = (int)(idx / (4 * npad));
+  float v[4];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int j = 8 * s + 2 * c + h;
+    const int g = j < npair ? pair[j].x : -1;
+    const float2 e = r < nat && g >= 0 ? eigr[(size_t)r * ngw + g] : make_float2(0.f, 0.f);
+    v[2 * h] = e.x;
+    v[2 * h + 1] = e.y;
+  }
+  unsigned char *hi = reinterpret_cast<unsigned char *>(etp + (size_t)s * npad * 32);
+  tc::st_split4(hi, hi + npad * 64, tc::core_off<kBK>(r, 4 * c), make_float4(v[0], v[1], v[2], v[3]));
+}
+// back-projection tiles per (128 pairs, 16 atoms), Re E then Im E
+__global__ void k_build_etb_pairs(const float2 *__restrict__ eigr, const int2 *__restrict__ pair,
+                                  int npair, int ngw, int nat, int nsa, int ngt,
+                                  float *__restrict__ etb) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (idx >= (long long)ngt * nsa * 512) return;
+  const int c = (int)(idx & 3);
+  const int gg = (int)((idx >> 2) & 127);
+  const int s = (int)((idx >> 9) % nsa);
+  const int t = (int)(idx / (512LL * nsa));
+  const int j = 128 * t + gg, g = j < npair ? pair[j].x : -1;
+  float re[4], im[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int a = 16 * s + 4 * c + q;
+    const float2 e = a < nat && g >= 0 ? eigr[(size_t)a * ngw + g] : make_float2(0.f, 0.f);
+    re[q] = e.x;
+    im[q] = e.y;
+  }
+  unsigned char *p = reinterpret_cast<unsigned char *>(etb + ((size_t)t * nsa + s) * 8192);
+  const uint32_t o = tc::core_off<kBK>(gg, 4 * c);
+  tc::st_split4(p, p + 8192, o, make_float4(re[0], re[1], re[2], re[3]));
+  tc::st_split4(p + 16384, p + 24576, o, make_float4(im[0], im[1], im[2], im[3]));
+}
+
 // ------------------------------------------------------------------ host side
 struct Shape {
   int L, per, nat, npad, nsa, nbt, ncolN, nbtiles;
@@ -574,10 +834,12 @@ struct Group {
   size_t etp_off, etb_off;
 };
 
-std::vector<Group> groups_of(const Projectors &P, int ngw_cell) {
+// over the cell's ngw G, or (fold) over its pairs
+std::vector<Group> groups_of(const Projectors &P, int ngw_cell, bool fold = false) {
   std::vector<Group> g;
-  const size_t nst = (size_t)(ngw_cell + kStepG - 1) / kStepG * (kStepG / 8);
-  const size_t ngt = (size_t)(ngw_cell + 127) / 128;
+  const int n = fold ? 8 * P.fold.groups : ngw_cell;
+  const size_t nst = (size_t)(n + kStepG - 1) / kStepG * (kStepG / 8);
+  const size_t ngt = (size_t)(n + 127) / 128;
   int atom0 = 0, p0 = 0;
   size_t eo = 0, bo = 0;
   for (int s = 0; s < (int)P.sp_na.size(); s++) {
@@ -585,7 +847,8 @@ std::vector<Group> groups_of(const Projectors &P, int ngw_cell) {
     if (na > 0 && L > 0) {
       g.push_back({s, atom0, na, L, p0, eo, bo});
       eo += nst * (size_t)((na + 15) / 16 * 16) * 32;  // npad x 128 bytes per 8 G
-      bo += ngt * (size_t)((na + 7) / 8) * 4096;       // 16 KB per (128 G, 8 atoms)
+      // 16 KB per (128 G, 8 atoms), 32 KB per (128 pairs, 16 atoms)
+      bo += fold ? ngt * (size_t)((na + 15) / 16) * 8192 : ngt * (size_t)((na + 7) / 8) * 4096;
     }
     atom0 += na;
     p0 += na * std::max(0, L);
@@ -639,10 +902,14 @@ int proj_tmem_cols(const Shape &s) {
   return tmem_cols(tmem_cols(s.npad) + 64 * proj_slots(s.npad));
 }
 
-int proj_smem(const Shape &s) {
+int proj_smem(const Shape &s, bool fold) {
   const int nbr_max = 127 / s.per + 2;
-  const int raw = round16(nbr_max * (kStepG + 1) * 8) + kStepG * 16;
+  const int raw = round16(nbr_max * raw_row(fold) * 8) + kStepG * 16;
   return block_smem(proj_slots(s.npad) * 2 * s.npad * 128 + kNR * raw, proj_tmem_cols(s));
+}
+
+int backpair_smem(const Shape &s) {
+  return block_smem(kNTB * (4 * kTileBytes128 + s.ncolN * 128), tmem_cols(2 * t2_col(s.ncolN)));
 }
 
 int back_smem(const Shape &s) {
@@ -660,9 +927,9 @@ int sm_count() {
 }
 
 // splits of the projection's K range: enough blocks to fill the GPU once
-int proj_splits(const Shape &s, int ngw, int nb, int *kg_out) {
+int proj_splits(const Shape &s, int ngw, int nb, int *kg_out, bool fold) {
   const int mt = (nb * s.per + 127) / 128;
-  const int smem = proj_smem(s);
+  const int smem = proj_smem(s, fold);
   const int per_sm = std::max(1, std::min(233472 / (smem + 1024), 512 / proj_tmem_cols(s)));
   int nsplit = std::max(1, std::min((ngw + 63) / 64, per_sm * sm_count() / mt));
   int kg = (ngw + nsplit - 1) / nsplit;
@@ -674,16 +941,18 @@ int proj_splits(const Shape &s, int ngw, int nb, int *kg_out) {
 template <int L>
 int launch_project(pspw_cell *c, const Shape &s, const float2 *psi, int ld, int ngw, int nb,
                    float *part, int nsplit, int kg, float *wt, const float *etp,
-                   const float *pkga, const float *pw) {
+                   const float *pkga, const float *pw, bool fold, unsigned odd) {
   const int mt = (nb * s.per + 127) / 128;
-  const int smem = proj_smem(s);
-  int rc = smem_allow_max(k_proj_tc<L>);
+  const int smem = proj_smem(s, fold);
+  auto kern = fold ? k_proj_tc<L, true> : k_proj_tc<L, false>;
+  int rc = smem_allow_max(kern);
   if (rc) return rc;
-  k_proj_tc<L><<<dim3(mt, nsplit), kThreadsP, smem, c->stream>>>(
-      psi, ld, ngw, nb, etp, pkga, s.nat, s.npad, kg, part, c->d_err);
-  const dim3 wgrid((4 * s.nsa + 31) / 32, s.nbtiles * s.nbt * L);
-  k_proj_tc_wtiles<L><<<wgrid, 32 * kWtWarps, 0, c->stream>>>(part, nsplit, nb, s.nat, pw, s.nbt,
-                                                               s.nsa, wt);
+  kern<<<dim3(mt, nsplit), kThreadsP, smem, c->stream>>>(
+      psi, ld, ngw, nb, etp, pkga, s.nat, s.npad, kg, part, c->d_err, c->proj.fold.d_pair, odd);
+  const int nsa = fold ? (s.nat + 15) / 16 : s.nsa;
+  const dim3 wgrid(((fold ? 8 : 4) * nsa + 31) / 32, s.nbtiles * s.nbt * L);
+  auto wkern = fold ? k_proj_tc_wtiles<L, true> : k_proj_tc_wtiles<L, false>;
+  wkern<<<wgrid, 32 * kWtWarps, 0, c->stream>>>(part, nsplit, nb, s.nat, pw, s.nbt, nsa, wt);
   c->kernel_launches += 2;
   PSPW_CUDA(cudaGetLastError());
   return PSPW_OK;
@@ -692,7 +961,20 @@ int launch_project(pspw_cell *c, const Shape &s, const float2 *psi, int ld, int 
 template <int L>
 int launch_back(pspw_cell *c, const Shape &s, const float *wt, const float *etb,
                 const float *pkga, int ngw, int nb, float2 *out, int ldo, const float2 *in,
-                int ldi, const float2 *xm2, int ldx, float a, float b, float g, bool pre) {
+                int ldi, const float2 *xm2, int ldx, float a, float b, float g, bool pre, bool fold,
+                unsigned odd) {
+  if (fold) {
+    const int npair = 8 * c->proj.fold.groups;
+    auto kern = pre ? k_backpair_tc<L, true> : k_backpair_tc<L, false>;
+    if (const int rc = smem_allow_max(kern)) return rc;
+    const dim3 grid((npair + 127) / 128, s.nbtiles);
+    kern<<<grid, kThreads, backpair_smem(s), c->stream>>>(
+        etb, wt, (s.nat + 15) / 16, npair, c->proj.fold.d_pair, odd, nb, s.nbt, pkga, out, ldo, in,
+        ldi, xm2, ldx, a, b, g, c->d_err);
+    c->kernel_launches++;
+    PSPW_CUDA(cudaGetLastError());
+    return PSPW_OK;
+  }
   const int smem = back_smem(s);
   auto kern = pre ? k_backproj_tc<L, true> : k_backproj_tc<L, false>;
   int rc = smem_allow_max(kern);
@@ -733,7 +1015,8 @@ int nl_tc_wait_check(pspw_cell *c, int complete) {
 bool nl_tc_usable(const pspw_cell *c) {
   static const bool off = std::getenv("PSPW_NL_SIMT") != nullptr;
   if (c->nl_path == PSPW_NL_SIMT || (off && c->nl_path != PSPW_NL_TENSOR_CORE)) return false;
-  return fits(c->proj) && c->proj.d_etp && c->proj.d_etb && c->d_err;
+  // (in the filter's stick order a cell with pair symmetry has no other tiles)
+  return fits(c->proj) && ((c->proj.d_etp && c->proj.d_etb) || c->proj.fold.ok) && c->d_err;
 }
 
 int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **etb) {
@@ -770,6 +1053,37 @@ int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **e
   return PSPW_OK;
 }
 
+int nl_tc_pair_tiles(pspw_cell *c) {
+  Projectors &P = c->proj;
+  Fold &f = P.fold;
+  if (f.etp) return PSPW_OK;
+  const int ngw = c->basis.ngw, n = 8 * f.groups;
+  const std::vector<Group> gs = groups_of(P, ngw, true);
+  const int nst = (n + kStepG - 1) / kStepG * (kStepG / 8), ngt = (n + 127) / 128;
+  size_t fe = 0, fb = 0;
+  for (const Group &g : gs) {
+    fe = g.etp_off + (size_t)nst * ((g.nat + 15) / 16 * 16) * 32;
+    fb = g.etb_off + (size_t)ngt * ((g.nat + 15) / 16) * 8192;
+  }
+  // one allocation: the projection tiles, then (16-byte aligned: whole tiles)
+  // the back-projection tiles
+  if (cudaMalloc(&f.etp, (fe + fb) * sizeof(float)) != cudaSuccess)
+    return fail(PSPW_ERR_OOM, "EIGR operand tiles");
+  f.etb = f.etp + fe;
+  for (const Group &g : gs) {
+    const int npad = (g.nat + 15) / 16 * 16, nsa = (g.nat + 15) / 16;
+    const float2 *e = P.d_eigr32 + (size_t)g.atom0 * ngw;
+    const long long n1 = (long long)nst * npad * 4, n2 = (long long)ngt * nsa * 512;
+    k_build_etp_pairs<<<(unsigned)((n1 + 255) / 256), 256, 0, c->stream>>>(
+        e, f.d_pair, n, ngw, g.nat, npad, nst, f.etp + g.etp_off);
+    k_build_etb_pairs<<<(unsigned)((n2 + 255) / 256), 256, 0, c->stream>>>(
+        e, f.d_pair, n, ngw, g.nat, nsa, ngt, f.etb + g.etb_off);
+    c->kernel_launches += 2;
+  }
+  PSPW_CUDA(cudaGetLastError());
+  return PSPW_OK;
+}
+
 int nl_tc_prepare(pspw_cell *c) {
   Projectors &P = c->proj;
   if (!fits(P) || P.d_etp) return PSPW_OK;
@@ -783,11 +1097,13 @@ size_t nl_tc_wtile_bytes(const pspw_cell *c, int nb) {
   return n;
 }
 
-int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, float **wt) {
+int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, float **wt,
+                  bool fold) {
   int ms = 1;
   for (const Group &g : groups_of(c->proj, c->basis.ngw)) {
     int kg = 0;
-    ms = std::max(ms, proj_splits(shape_of(g, nb), ngw, nb, &kg));
+    ms = std::max(ms, proj_splits(shape_of(g, nb), fold ? 8 * c->proj.fold.groups : ngw, nb, &kg,
+                                  fold));
   }
   // the partial sums of any one species fit max_split x 2 nb nproj floats
   int rc = ws_reserve(c, kWsProjPart, sizeof(float) * (size_t)ms * 2 * nb * c->proj.nproj,
@@ -800,29 +1116,42 @@ int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, f
 }
 
 int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, float *part,
-                  int max_split, float *wt) {
+                  int max_split, float *wt, bool fold) {
   const Projectors &P = c->proj;
+  const int nk = fold ? 8 * P.fold.groups : ngw;  // pairs or G to sum over
   const size_t cap = (size_t)std::max(1, max_split) * 2 * nb * P.nproj;  // floats of part
   size_t woff = 0;
-  for (const Group &g : groups_of(P, c->basis.ngw)) {
+  for (const Group &g : groups_of(P, c->basis.ngw, fold)) {
     const Shape s = shape_of(g, nb);
     int kg = 0;
-    int nsplit = proj_splits(s, ngw, nb, &kg);
+    int nsplit = proj_splits(s, nk, nb, &kg, fold);
     const int lim = (int)std::max<size_t>(1, cap / ((size_t)nb * s.per * s.nat));
     if (nsplit > lim) {
       nsplit = lim;
-      kg = ((ngw + nsplit - 1) / nsplit + kStepG - 1) / kStepG * kStepG;
-      nsplit = (ngw + kg - 1) / kg;
+      kg = ((nk + nsplit - 1) / nsplit + kStepG - 1) / kStepG * kStepG;
+      nsplit = (nk + kg - 1) / kg;
     }
     float *w = wt + woff / sizeof(float);
-    const float *etp = P.d_etp + g.etp_off, *pk = P.d_pkga32 + (size_t)g.sp * c->basis.ngw * 4,
+    const float *etp = (fold ? P.fold.etp : P.d_etp) + g.etp_off, *pk = P.d_pkga32 + (size_t)g.sp * c->basis.ngw * 4,
                 *pw = P.d_pw32 + g.p0;
+    const unsigned odd = fold ? P.sp_odd[g.sp] : 0u;
     int rc;
     switch (s.L) {
-      case 1: rc = launch_project<1>(c, s, psi, ld, ngw, nb, part, nsplit, kg, w, etp, pk, pw); break;
-      case 2: rc = launch_project<2>(c, s, psi, ld, ngw, nb, part, nsplit, kg, w, etp, pk, pw); break;
-      case 3: rc = launch_project<3>(c, s, psi, ld, ngw, nb, part, nsplit, kg, w, etp, pk, pw); break;
-      default: rc = launch_project<4>(c, s, psi, ld, ngw, nb, part, nsplit, kg, w, etp, pk, pw);
+      case 1:
+        rc = launch_project<1>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+                                etp, pk, pw, fold, odd);
+        break;
+      case 2:
+        rc = launch_project<2>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+                                etp, pk, pw, fold, odd);
+        break;
+      case 3:
+        rc = launch_project<3>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+                                etp, pk, pw, fold, odd);
+        break;
+      default:
+        rc = launch_project<4>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+                                etp, pk, pw, fold, odd);
     }
     if (rc) return rc;
     woff += group_wtile_bytes(s);
@@ -832,23 +1161,35 @@ int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, floa
 
 int nl_tc_backproject(pspw_cell *c, const float *wt, int ngw, int nb, float2 *out, int ldo,
                       const float2 *in, int ldi, const float2 *xm2, int ldx, float a, float b,
-                      float g, bool pre) {
+                      float g, bool pre, bool fold) {
   const Projectors &P = c->proj;
   size_t woff = 0;
   bool first = true;
-  for (const Group &gp : groups_of(P, c->basis.ngw)) {
+  for (const Group &gp : groups_of(P, c->basis.ngw, fold)) {
     const Shape s = shape_of(gp, nb);
     const float *w = wt + woff / sizeof(float);
-    const float *etb = P.d_etb + gp.etb_off, *pk = P.d_pkga32 + (size_t)gp.sp * c->basis.ngw * 4;
+    const float *etb = (fold ? P.fold.etb : P.d_etb) + gp.etb_off, *pk = P.d_pkga32 + (size_t)gp.sp * c->basis.ngw * 4;
     // the first species applies the recurrence's update; the others add
     // their a * sum to it (the `pre` form)
     const bool pr = first ? pre : true;
+    const unsigned odd = fold ? P.sp_odd[gp.sp] : 0u;
     int rc;
     switch (s.L) {
-      case 1: rc = launch_back<1>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi, xm2, ldx, a, b, g, pr); break;
-      case 2: rc = launch_back<2>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi, xm2, ldx, a, b, g, pr); break;
-      case 3: rc = launch_back<3>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi, xm2, ldx, a, b, g, pr); break;
-      default: rc = launch_back<4>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi, xm2, ldx, a, b, g, pr);
+      case 1:
+        rc = launch_back<1>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi,
+                            xm2, ldx, a, b, g, pr, fold, odd);
+        break;
+      case 2:
+        rc = launch_back<2>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi,
+                            xm2, ldx, a, b, g, pr, fold, odd);
+        break;
+      case 3:
+        rc = launch_back<3>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi,
+                            xm2, ldx, a, b, g, pr, fold, odd);
+        break;
+      default:
+        rc = launch_back<4>(c, s, w, etb, pk, ngw, nb, out, ldo, in, ldi,
+                            xm2, ldx, a, b, g, pr, fold, odd);
     }
     if (rc) return rc;
     woff += group_wtile_bytes(s);

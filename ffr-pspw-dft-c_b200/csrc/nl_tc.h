@@ -16,24 +16,30 @@ int nl_tc_prepare(pspw_cell *c);
 // The same tiles from a given EIGR copy (FP32, [nat][ngw]) into new buffers.
 int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **etb);
 
+// The tiles over pairs (+G, -G) of the cell's current G order (its fold must
+// be ok), built on the first call of each order.
+int nl_tc_pair_tiles(pspw_cell *c);
+
 // Bytes of the projection operand tiles for nb bands.
 size_t nl_tc_wtile_bytes(const pspw_cell *c, int nb);
 
 // Scratch of nl_tc_project from the cell's workspaces: partial sums (at most
 // *max_split slices) and the projection operand tiles.
-int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, float **wt);
+int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, float **wt,
+                  bool fold);
 
 // Projections of nb bands (first ngw G) into the operand tiles `wt`:
 // W(a,lm,b) = WNL(lm) sum_G conj(EIGR(G,a)) PKG_A(lm,G) psi_b(G).
+// fold (in all three): over pairs, after nl_tc_pair_tiles.
 int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, float *part,
-                  int max_split, float *wt);
+                  int max_split, float *wt, bool fold);
 
 // out = a*(out + sum_{a,lm} EIGR PKG_A W) + b*in + g*xm2 on the first ngw G;
 // with pre, out already holds a*(H_loc psi) + b*in + g*xm2 and the kernel
 // adds a * sum EIGR PKG_A W.
 int nl_tc_backproject(pspw_cell *c, const float *wt, int ngw, int nb, float2 *out, int ldo,
                       const float2 *in, int ldi, const float2 *xm2, int ldx, float a, float b,
-                      float g, bool pre = false);
+                      float g, bool pre, bool fold);
 
 // Runs one bounded device-side barrier wait on the cell stream and returns
 // the cell's status after it: PSPW_ERR_TIMEOUT when the barrier is never
