@@ -38,11 +38,38 @@ __host__ __device__ __forceinline__ double2 operator-(double2 a, double2 b) {
 __host__ __device__ __forceinline__ double2 operator*(double s, double2 a) {
   return make_double2(s * a.x, s * a.y);
 }
+// FP32 pairs add in one instruction (add.f32x2, each half rounded as a scalar
+// add): the DFT butterflies are mostly complex adds, and the plane kernels
+// issue-bound beside their shared-memory traffic.
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_of(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+#endif
 __host__ __device__ __forceinline__ float2 operator+(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+#else
   return make_float2(a.x + b.x, a.y + b.y);
+#endif
 }
 __host__ __device__ __forceinline__ float2 operator-(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+#else
   return make_float2(a.x - b.x, a.y - b.y);
+#endif
 }
 __host__ __device__ __forceinline__ float2 operator*(float s, float2 a) {
   return make_float2(s * a.x, s * a.y);
