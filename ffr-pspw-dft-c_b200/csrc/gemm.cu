@@ -442,10 +442,15 @@ static int launch_dmma(pspw_cell *c, bool conj, int m, int n, int k, double2 alp
   cudaStream_t st = c->stream;
   const int mt = (m + D::BM - 1) / D::BM, nt = (n + D::BN - 1) / D::BN;
   // K split over blocks when the output has fewer blocks than the SMs hold
+  // (kZgemmUpperC: the tiles below the diagonal end at once and do not count)
   const int target = D::MIN_BLOCKS * sm_count_now();
+  int tiles = mt * nt;
+  if (tri == kZgemmUpperC)
+    for (int i = 0; i < mt; i++)
+      for (int j = 0; j < nt; j++) tiles -= i * D::BM >= (j + 1) * D::BN;
   int nsplit = 1;
-  if (k > 8 * D::BK && mt * nt < target)
-    nsplit = std::max(1, std::min((k + 255) / 256, (target + mt * nt - 1) / (mt * nt)));
+  if (k > 8 * D::BK && tiles < target)
+    nsplit = std::max(1, std::min((k + 255) / 256, (target + tiles - 1) / tiles));
   int kchunk = k > 0 ? (k + nsplit - 1) / nsplit : D::BK;
   kchunk = (kchunk + D::BK - 1) / D::BK * D::BK;
   nsplit = k > 0 ? (k + kchunk - 1) / kchunk : 1;

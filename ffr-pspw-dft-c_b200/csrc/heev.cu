@@ -894,15 +894,63 @@ __global__ void __launch_bounds__(32 * kBTWarps) k_back_tr(const double2 *__rest
 // L = U^H packed row-major into Lg, stat[0] = 0 or k + 1 when the k-th pivot
 // is not positive, stat[1] = max |U_kk| / min |U_kk|.  Works on L packed in
 // shared memory; k_tri_inv then forms U^-1 on many blocks.
+//
+// mode kCholScaled: the factor is that of D G D with D = diag(G)^-1/2, the
+// Gram matrix of the columns scaled to unit norm, and scale[i] = D_ii (a
+// column that is zero, or whose squared norm is too small or large to hold
+// its digits, counts as a failed pivot).
+// mode kCholNear: when max |G - I| < 1e-9 no factorisation is needed: stat[1]
+// = -1 and k_tri_inv takes U^-1 to first order in G - I, whose square is
+// below n * 1e-18.  The second pass of CholeskyQR2 ends so unless the block
+// was ill-conditioned; its factorisation and inverse took 165 + 33 us at
+// order 146, this check 6 us.
+constexpr int kCholPlain = 0, kCholScaled = 1, kCholNear = 2;
 __global__ void __launch_bounds__(kT1, 1)
     k_chol_inv(const double2 *__restrict__ G, int ldg, int n, double2 *__restrict__ Lg,
-               double *__restrict__ stat) {
+               double *__restrict__ stat, int mode, double *__restrict__ scale) {
   extern __shared__ double2 L[];
   __shared__ int s_failed;
+  __shared__ double s_d[kHeevMax];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  for (int i = warp; i < n; i += nw)
-    for (int j = lane; j <= i; j += 32) L[lp(i, j)] = cconj(G[j + (size_t)i * ldg]);
   if (tid == 0) s_failed = 0;
+  __syncthreads();
+  if (mode == kCholNear) {
+    int far = 0;
+    for (int i = warp; i < n; i += nw)
+      for (int j = lane; j <= i; j += 32) {
+        const double2 g = G[j + (size_t)i * ldg];
+        const double a = fabs(i == j ? g.x - 1.0 : g.x), b = fabs(g.y);
+        far |= !(a < 1e-9 && b < 1e-9);
+      }
+    if (!__syncthreads_or(far)) {
+      if (tid == 0) {
+        stat[0] = 0.0;
+        stat[1] = -1.0;
+      }
+      return;
+    }
+  }
+  if (mode == kCholScaled) {
+    for (int i = tid; i < n; i += blockDim.x) {
+      const double g = G[i + (size_t)i * ldg].x;
+      const bool ok = g > 1e-200 && g < 1e200;
+      if (!ok) s_failed = i + 1;
+      s_d[i] = ok ? 1.0 / sqrt(g) : 1.0;
+      scale[i] = s_d[i];
+    }
+    __syncthreads();
+  }
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j <= i; j += 32) {
+      double2 g = cconj(G[j + (size_t)i * ldg]);
+      if (mode == kCholScaled) {
+        g = i == j ? make_double2(1.0, 0.0)
+                   : make_double2(s_d[i] * s_d[j] * g.x, s_d[i] * s_d[j] * g.y);
+      }
+      L[lp(i, j)] = g;
+    }
+  __syncthreads();
+  const int bad = s_failed;  // a norm out of range, before warp 0 may set it below
   __syncthreads();
   // blocked right-looking Cholesky with panels of kCB columns: warp 0
   // factors the panel's kCB x kCB diagonal block (warp-synchronous steps),
@@ -911,7 +959,7 @@ __global__ void __launch_bounds__(kT1, 1)
   // three barriers per panel
   __shared__ double s_idk[kCB];
   double dmax = 0.0, dmin = INFINITY;  // kept by thread 0
-  for (int k0 = 0; k0 < n; k0 += kCB) {
+  for (int k0 = bad ? n : 0; k0 < n; k0 += kCB) {
     const int k1 = min(n, k0 + kCB);
     if (warp == 0) {
       for (int k = k0; k < k1; k++) {
@@ -1028,15 +1076,30 @@ __global__ void __launch_bounds__(kT1, 1)
 // M = L^-1 by forward substitution: lane l keeps the running sums
 // s_i = sum_{k=j}^{i-1} L(i, k) M(k, j) of rows i = l (mod 32) in registers,
 // M(k, j) = -(1 / L(k, k)) s_k is broadcast from its owner and added into
-// the rows below.  Uinv(r, c) = conj(M(c, r)) for r <= c, 0 below.  Nothing
-// is written when the factorisation failed (stat[0] != 0).
+// the rows below.  Uinv(r, c) = conj(M(c, r)) for r <= c, 0 below, row r times
+// scale[r] when given (then X Uinv = (X D)(D G D's U^-1)).  Nothing is written
+// when the factorisation failed (stat[0] != 0); with stat[1] = -1, Uinv = I -
+// strict upper(G) - diag(G - I) / 2.
 constexpr int kInvWarps = 4;
 __global__ void __launch_bounds__(32 * kInvWarps) k_tri_inv(const double2 *__restrict__ Lg, int n,
                                                            double2 *__restrict__ Uinv, int ldu,
-                                                           const double *__restrict__ stat) {
+                                                           const double *__restrict__ stat,
+                                                           const double *__restrict__ scale,
+                                                           const double2 *__restrict__ G,
+                                                           int ldg) {
   extern __shared__ double2 Ls[];  // packed rows j0..n-1
   __shared__ double dinv[kHeevMax];
   if (stat[0] != 0.0) return;  // uniform
+  if (stat[1] == -1.0) {
+    const int j1 = min(n, (int)(blockIdx.x + 1) * kInvWarps);
+    for (int e = blockIdx.x * kInvWarps * n + threadIdx.x; e < j1 * n; e += blockDim.x) {
+      const int c = e / n, r = e - c * n;
+      const double2 g = r <= c ? G[r + (size_t)c * ldg] : make_double2(0.0, 0.0);
+      Uinv[(size_t)c * ldu + r] = r == c ? make_double2(1.0 - 0.5 * (g.x - 1.0), 0.0)
+                                         : make_double2(-g.x, -g.y);
+    }
+    return;
+  }
   const int j0 = blockIdx.x * kInvWarps, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int base = lp(j0, 0), np = n * (n + 1) / 2;
@@ -1046,6 +1109,7 @@ __global__ void __launch_bounds__(32 * kInvWarps) k_tri_inv(const double2 *__res
   __syncthreads();
   const int j = j0 + warp;
   if (j >= n) return;  // whole warp
+  const double sj = scale ? scale[j] : 1.0;
   double2 sacc[kColsL];
   int ro[kColsL];  // lp(i, 0) - base of the lane's rows
 #pragma unroll
@@ -1066,7 +1130,10 @@ __global__ void __launch_bounds__(32 * kInvWarps) k_tri_inv(const double2 *__res
                    sy = __shfl_sync(0xffffffffu, sacc[kb].y, kl);
       const double di = dinv[k];
       const double2 mk = k == j ? make_double2(di, 0.0) : make_double2(-di * sx, -di * sy);
-      if (lane == 0) Uinv[(size_t)k * ldu + j] = cconj(mk);
+      if (lane == 0) {
+        const double2 u = cconj(mk);
+        Uinv[(size_t)k * ldu + j] = make_double2(sj * u.x, sj * u.y);
+      }
       if (lane > kl && lane + 32 * kb < n) sacc[kb] = cfma_(Ls[ro[kb] + k], mk, sacc[kb]);
 #pragma unroll
       for (int q = kb + 1; q < kColsL; q++)
@@ -1114,7 +1181,7 @@ int dev_heev_small(pspw_cell *c, double2 *A, int lda, double *w, int n, void *wo
 }
 
 int dev_chol_inv_upper(pspw_cell *c, const double2 *G, int ldg, int n, double2 *Uinv, int ldu,
-                       double *stat) {
+                       double *stat, double *scale, bool near_identity) {
   if (n < 1 || n > kHeevMax || ldg < n || ldu < n)
     return fail(PSPW_ERR_ARG, "chol_inv_upper: n must be in 1.." + std::to_string(kHeevMax));
   const int np = n * (n + 1) / 2;
@@ -1123,9 +1190,10 @@ int dev_chol_inv_upper(pspw_cell *c, const double2 *G, int ldg, int n, double2 *
   int rc;
   if ((rc = ws_reserve(c, kWsChol, sizeof(double2) * (size_t)np, (void **)&Lg))) return rc;
   if ((rc = smem_allow_max(k_chol_inv)) || (rc = smem_allow_max(k_tri_inv))) return rc;
-  k_chol_inv<<<1, kT1, smem, c->stream>>>(G, ldg, n, Lg, stat);
-  k_tri_inv<<<(n + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, smem, c->stream>>>(Lg, n, Uinv,
-                                                                               ldu, stat);
+  const int mode = near_identity ? kCholNear : (scale ? kCholScaled : kCholPlain);
+  k_chol_inv<<<1, kT1, smem, c->stream>>>(G, ldg, n, Lg, stat, mode, scale);
+  k_tri_inv<<<(n + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, smem, c->stream>>>(
+      Lg, n, Uinv, ldu, stat, mode == kCholScaled ? scale : nullptr, G, ldg);
   c->kernel_launches += 2;
   PSPW_CUDA(cudaGetLastError());
   return PSPW_OK;

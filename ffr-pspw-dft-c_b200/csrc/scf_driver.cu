@@ -50,21 +50,6 @@ __global__ void k_real_to_z(const double *__restrict__ a, double2 *b, int k, int
   b[i] = make_double2(r <= col ? a[r + (size_t)lda * col] : 0.0, 0.0);
 }
 
-// column j of X (m rows, ld) scaled by 1/sqrt(d[j]) where d[j] > 0
-__global__ void k_unit_cols(double2 *X, int ld, int m, int n, const double *__restrict__ d) {
-  const size_t tot = (size_t)m * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e / m), i = (int)(e - (size_t)j * m);
-    const double dj = d[j];
-    if (dj > 0.0) {
-      const double s = 1.0 / sqrt(dj);
-      double2 *p = X + (size_t)j * ld + i;
-      *p = make_double2(s * p->x, s * p->y);
-    }
-  }
-}
-
 // ChebySCFLoop.cpp:7-34: |A v1|^2 with v1 = 1/sqrt(N) (ones), A the leading
 // N x N block of the lda-strided matrix
 double induced_norm_mat(const double *A, int lda, int N) {
@@ -89,32 +74,30 @@ double induced_norm_mat(const double *A, int lda, int N) {
 // below 1/sqrt(eps); the ratio of the largest to the smallest diagonal of
 // the first U bounds cond(X) from below, and above 1e6 (or when the
 // factorisation fails) the block goes to the Householder QR instead.  The
-// columns are first scaled to unit norm (the span is unchanged): the filter
-// multiplies the eigen-components of its block by factors that span orders
-// of magnitude, so the filtered columns are nearly orthogonal but of very
-// different lengths, an ill-conditioning that the scaling removes.
+// first factorisation is that of the Gram matrix scaled to a unit diagonal
+// (the span is unchanged): the filter multiplies the eigen-components of its
+// block by factors that span orders of magnitude, so the filtered columns are
+// nearly orthogonal but of very different lengths, an ill-conditioning that
+// the scaling removes.  The norms are the Gram matrix's diagonal and the
+// scaling goes into the rows of U^-1, so X itself is not touched (its own two
+// passes, norms and scaling, took 38 us of a 975 us call on Si64).
 // Both passes are enqueued before the host reads the two pivot statuses
 // (one synchronisation): the first pass writes W only, so X is intact for
 // the Householder fallback, and a failed first factorisation leaves U as it
 // was, which only makes the second pass's numbers meaningless.
 // G, U: n x n scratch (ld n); dn: n doubles; stat: 4 doubles; W: ngw x n.
+// n > kHeevMax is beyond the one-block factorisation: Householder.
 int span_orthonormalize(pspw_cell *c, double2 *X, int ngw, int n, double2 *G, double2 *U,
                         double *dn, double *stat, double2 *W, int *info) {
   const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
   int rc;
-  if ((rc = dev_coldot(c, X, ngw, X, ngw, ngw, n, dn))) return rc;
-  k_unit_cols<<<4 * 148, 256, 0, c->stream>>>(X, ngw, ngw, n, dn);
-  c->kernel_launches++;
-  PSPW_CUDA(cudaGetLastError());
-  if (n > kHeevMax) {  // beyond the one-block factorisation: Householder
-    return dev_ortho_qr(c, X, ngw, ngw, n, info);
-  }
+  if (n > kHeevMax) return dev_ortho_qr(c, X, ngw, ngw, n, info);
   for (int pass = 0; pass < 2; pass++) {
     double2 *src = pass == 0 ? X : W;
     // the factorisation reads the upper triangle of G only
     if ((rc = zgemm_tri(c, 'C', kZgemmUpperC, n, n, ngw, one, src, ngw, src, ngw, zero, G, n)))
       return rc;
-    if ((rc = dev_chol_inv_upper(c, G, n, n, U, n, stat + 2 * pass))) return rc;
+    if ((rc = dev_chol_inv_upper(c, G, n, n, U, n, stat + 2 * pass, dn, pass == 1))) return rc;
     // U^-1 is upper triangular (zeros stored below the diagonal)
     if (pass == 0 &&
         (rc = zgemm_tri(c, 'N', kZgemmUpperB, ngw, n, n, one, X, ngw, U, n, zero, W, ngw)))
