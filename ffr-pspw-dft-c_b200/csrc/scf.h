@@ -3,6 +3,8 @@
 // with the local-potential data and the mixing history kept on the device.
 #pragma once
 
+#include <functional>
+
 #include <vector>
 
 #include "engine.h"
@@ -49,5 +51,13 @@ int xc_pz_dev(pspw_scf *s, const double *d_rho, double *d_vxc, double *exc);
 int normalize_rho_dev(pspw_scf *s, double *d_rho, double omega, double nel, int *warn);
 int kerker_prec_dev(pspw_scf *s, double *d_x, double beta, double q0);
 int mix_dev(pspw_scf *s, int iter, double *d_rhoe, double *d);
+
+// pspw_cheby_scf (pspw_gpu.h) with the start block asked for when the loop
+// needs it, after the first Lanczos bounds (params->idiag < 0 only), and the
+// final block copied out only where X_out is given.
+int cheby_scf_run(pspw_scf *s, const pspw_scf_params *p, const double *focc,
+                  const double *rho_start, const double *v0,
+                  const std::function<const double *()> &start_block, double *X_out, double *eig,
+                  double *rho_out, double *hist, int *iterations, int *converged, double *e6);
 
 }  // namespace pspw

@@ -18,6 +18,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -177,13 +178,13 @@ void fermi_occupations(const double *eig, int nx, double nel, double w, double e
 }  // namespace
 }  // namespace pspw
 
-using namespace pspw;
+namespace pspw {
 
-extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const double *focc,
-                              const double *rho_start, const double *v0, double *X_io,
-                              double *eig, double *rho_out, double *hist, int *iterations,
-                              int *converged, double *e6) {
-  if (!s || !p || !focc || !rho_start || !v0 || !X_io || !eig || !iterations || !converged || !e6)
+int cheby_scf_run(pspw_scf *s, const pspw_scf_params *p, const double *focc,
+                  const double *rho_start, const double *v0,
+                  const std::function<const double *()> &start_block, double *X_out, double *eig,
+                  double *rho_out, double *hist, int *iterations, int *converged, double *e6) {
+  if (!s || !p || !focc || !rho_start || !v0 || !eig || !iterations || !converged || !e6)
     return fail(PSPW_ERR_ARG, "cheby_scf: null argument");
   pspw_cell *c = s->cell;
   PSPW_CUDA(cudaSetDevice(c->device));
@@ -215,7 +216,7 @@ extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const doubl
   if (!mem.get(&X, (size_t)ngw * nx2) || !mem.get(&dcn, nx2) || !mem.get(&HX, (size_t)ngw * nx2) ||
       !mem.get(&T, (size_t)nx2 * nx2) || !mem.get(&dU, (size_t)nx2 * nx2) ||
       !mem.get(&dstat, 4) || !mem.get(&dv0, ngw) || !mem.get(&df, ngw) ||
-      !mem.get(&dRT, (size_t)k * k) || !mem.get(&veff, nnr) || !mem.get(&rho, nnr) ||
+      !mem.get(&dRT, k <= kTriEigMax ? 1 : (size_t)k * k) || !mem.get(&veff, nnr) || !mem.get(&rho, nnr) ||
       !mem.get(&wT, std::max(k, nx2)) || !mem.get(&dprec, ngw) ||
       (fprec == PSPW_PREC_F32 && !mem.get(&Xf, (size_t)ngw * nx2)))
     return fail(PSPW_ERR_OOM, "cheby_scf: device memory");
@@ -241,7 +242,21 @@ extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const doubl
   // the bounds only shape the filter, so in the mixed mode their H*v
   // products run in the filter's precision
   if ((rc = lanczos_dev(c, dv0, ngw, k, rT.data(), k, df, fprec))) return rc;
-  {
+  if (k <= kTriEigMax) {
+    // T is tridiagonal up to the rounding that the reorthogonalisation
+    // leaves, so its eigenvalues come from the bisection of the own kernel
+    // (the reference's dsyev, and before that zheevd of order 284 here, works
+    // on the full matrix)
+    std::vector<double> de(2 * (size_t)k, 0.0);
+    for (int i = 0; i < k; i++) de[i] = rT[(size_t)i * k + i];
+    for (int i = 0; i + 1 < k; i++) de[k + i] = rT[(size_t)(i + 1) * k + i];
+    double *d_de;
+    if (!mem.get(&d_de, 2 * (size_t)k)) return fail(PSPW_ERR_OOM, "cheby_scf: device memory");
+    PSPW_CUDA(cudaMemcpyAsync(d_de, de.data(), sizeof(double) * 2 * k, cudaMemcpyHostToDevice, st));
+    if ((rc = dev_tri_eigvals(c, d_de, d_de + k, k, wT))) return rc;
+    PSPW_CUDA(cudaMemcpyAsync(evT.data(), wT, sizeof(double) * k, cudaMemcpyDeviceToHost, st));
+    PSPW_CUDA(cudaStreamSynchronize(st));
+  } else {
     double *dr;
     if (!mem.get(&dr, (size_t)k * k)) return fail(PSPW_ERR_OOM, "cheby_scf: device memory");
     PSPW_CUDA(cudaMemcpyAsync(dr, rT.data(), sizeof(double) * k * k, cudaMemcpyHostToDevice, st));
@@ -295,7 +310,9 @@ extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const doubl
   };
   if (p->idiag < 0) {
     // the caller's random block, orthonormalised (ChebySCFLoop.cpp:201-209)
-    PSPW_CUDA(cudaMemcpyAsync(X, X_io, sizeof(double2) * (size_t)ngw * nx2, cudaMemcpyHostToDevice,
+    const double *x0 = start_block();
+    if (!x0) return fail(PSPW_ERR_ARG, "cheby_scf: null argument");
+    PSPW_CUDA(cudaMemcpyAsync(X, x0, sizeof(double2) * (size_t)ngw * nx2, cudaMemcpyHostToDevice,
                               st));
     int info = 0;
     if ((rc = dev_ortho_qr(c, X, ngw, ngw, nx2, &info))) return rc;
@@ -382,14 +399,29 @@ extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const doubl
   }
   // results
   for (int i = 0; i < nx; i++) eig[i] = evals[i];
-  PSPW_CUDA(cudaMemcpyAsync(X_io, X, sizeof(double2) * (size_t)ngw * nx2, cudaMemcpyDeviceToHost,
-                            st));
+  if (X_out)
+    PSPW_CUDA(cudaMemcpyAsync(X_out, X, sizeof(double2) * (size_t)ngw * nx2,
+                              cudaMemcpyDeviceToHost, st));
   if (rho_out)
     PSPW_CUDA(cudaMemcpyAsync(rho_out, rho, sizeof(double) * nnr, cudaMemcpyDeviceToHost, st));
   PSPW_CUDA(cudaStreamSynchronize(st));
   for (int i = 0; i < 6; i++) e6[i] = en[i];
   *iterations = done_iters;
   return device_status(c);
+}
+
+}  // namespace pspw
+
+using namespace pspw;
+
+extern "C" int pspw_cheby_scf(pspw_scf *s, const pspw_scf_params *p, const double *focc,
+                              const double *rho_start, const double *v0, double *X_io,
+                              double *eig, double *rho_out, double *hist, int *iterations,
+                              int *converged, double *e6) {
+  if (!X_io) return fail(PSPW_ERR_ARG, "cheby_scf: null argument");
+  return cheby_scf_run(
+      s, p, focc, rho_start, v0, [&] { return X_io; }, X_io, eig, rho_out, hist, iterations,
+      converged, e6);
 }
 
 extern "C" int pspw_ortho_span_dev(pspw_cell *c, double *d_X, int ngw, int n) {
