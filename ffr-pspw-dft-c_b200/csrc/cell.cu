@@ -242,8 +242,7 @@ int pspw_cell_destroy(pspw_cell *c) {
                   B.d_xa_of_x, B.d_kin64, B.d_kin32, B.d_xkg64, c->proj.d_eigr64, c->proj.d_eigr32,
                   c->proj.d_pkga64, c->proj.d_pkga32, c->proj.d_patom, c->proj.d_psp,
                   c->proj.d_plm, c->proj.d_pw64, c->proj.d_pw32, c->d_veff64, c->d_veff32,
-                  B.d_col_x, B.d_col_y, B.d_pinv[0], B.d_pinv[1], B.d_pinv[2], c->d_vperm64,
-                  c->d_vperm32, c->proj.d_etp, c->proj.d_etb, B.d_wgrid, c->proj.d_beta64,
+                  B.d_col_x, c->d_vperm64, c->proj.d_etp, c->proj.d_etb, B.d_wgrid, c->proj.d_beta64,
                   c->stick.sg_ig, c->stick.kin64, c->stick.kin32, c->stick.eigr64,
                   c->stick.eigr32, c->stick.pkga64, c->stick.pkga32, c->stick.etp,
                   c->stick.etb, c->stick.beta64, c->proj.fold_mem,
@@ -440,16 +439,22 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
   // register-FFT path when all three lengths split into two register DFTs
   set_fft_paths(&B);
   if (B.fast32) {
-    if ((rc = upload(&B.d_col_x, col_x)) || (rc = upload(&B.d_col_y, col_y))) return bail(rc);
+    // one table and one allocation each: col_x, col_y, the three orders; the
+    // permuted potential in both precisions
+    std::vector<int> tab(col_x);
+    tab.insert(tab.end(), col_y.begin(), col_y.end());
     for (int i = 0; i < 3; i++) {
       const Split &sp = B.split[i];
-      std::vector<int> pinv(nr[i]);
-      for (int p = 0; p < nr[i]; p++) pinv[p] = p / sp.a + sp.b * (p % sp.a);
-      if ((rc = upload(&B.d_pinv[i], pinv))) return bail(rc);
+      for (int p = 0; p < nr[i]; p++) tab.push_back(p / sp.a + sp.b * (p % sp.a));
     }
-    if (cudaMalloc(&c->d_vperm64, (size_t)B.nnr * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&c->d_vperm32, (size_t)B.nnr * sizeof(float)) != cudaSuccess)
+    if ((rc = upload(&B.d_col_x, tab))) return bail(rc);
+    B.d_col_y = B.d_col_x + ncol;
+    B.d_pinv[0] = B.d_col_y + ncol;
+    B.d_pinv[1] = B.d_pinv[0] + nr1;
+    B.d_pinv[2] = B.d_pinv[1] + nr2;
+    if (cudaMalloc(&c->d_vperm64, (size_t)B.nnr * (sizeof(double) + sizeof(float))) != cudaSuccess)
       return bail(fail(PSPW_ERR_OOM, "cell_create: permuted V_eff"));
+    c->d_vperm32 = reinterpret_cast<float *>(c->d_vperm64 + B.nnr);
   }
   // ---- projectors, species-major then atom then lm (ApplyHam_block.cpp:68-117)
   Projectors &P = c->proj;

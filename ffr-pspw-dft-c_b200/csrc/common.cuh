@@ -39,8 +39,8 @@ __host__ __device__ __forceinline__ double2 operator*(double s, double2 a) {
   return make_double2(s * a.x, s * a.y);
 }
 // FP32 pairs add in one instruction (add.f32x2, each half rounded as a scalar
-// add): the DFT butterflies are mostly complex adds, and the plane kernels
-// issue-bound beside their shared-memory traffic.
+// add): the DFT butterflies are mostly complex adds, and every FFT kernel
+// issues at 60-75 % of its slots.  FP32 filter of Si64 3.03 -> 2.95 ms.
 #ifdef __CUDA_ARCH__
 __device__ __forceinline__ unsigned long long f2_bits(float2 a) {
   unsigned long long r;

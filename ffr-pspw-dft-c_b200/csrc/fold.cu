@@ -244,7 +244,7 @@ __global__ void k_fold_reduce(const double2 *__restrict__ part, int nsplit, int 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double2 s = part[i];
-#pragma unroll 4
+#pragma unroll 8
   for (int k = 1; k < nsplit; k++) s = s + part[(size_t)k * n + i];
   const int p = i % nproj;
   if (w) s = make_double2(w[p] * s.x, w[p] * s.y);
@@ -519,8 +519,9 @@ int launch_proj(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, c
       f.d_b64, f.d_pair, f.groups, P.nproj, psi, ld, nb, gchunk, w, P.d_odd, wp, part);
   c->kernel_launches++;
   if (nsplit > 1) {
-    k_fold_reduce<<<(nb * P.nproj + 255) / 256, 256, 0, c->stream>>>(part, nsplit, nb, P.nproj, w,
-                                                                    P.d_odd, wp);
+    // small blocks: few outputs with many slices spread over more SMs
+    k_fold_reduce<<<(nb * P.nproj + 63) / 64, 64, 0, c->stream>>>(part, nsplit, nb, P.nproj, w,
+                                                                 P.d_odd, wp);
     c->kernel_launches++;
   }
   PSPW_CUDA(cudaGetLastError());
