@@ -242,51 +242,49 @@ constexpr size_t plane_rho_smem() {
   return plane_rho_acc_off<NX, NY, T>() + sizeof(double) * (size_t)NX * NY;
 }
 
-// The y steps run on the compact view of the active columns, as in k_plane;
-// only that view is cleared per band.
+// (Full rows throughout: the compact y view of k_plane, whose first x step
+// holds two items of eight complex values over a barrier, took 512 against 433
+// us for the density of Si64.)
 template <int NX, int NY, typename T>
 __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NT) k_plane_rho(
     FastGeo g, int n3, const T *__restrict__ wx_g, const T *__restrict__ wy_g,
     const T *__restrict__ S, int nbb, int bands_per_group, const double *__restrict__ wband,
     double *__restrict__ part) {
-  constexpr int LS = PlaneCfg<NX, NY>::LS, NT = PlaneCfg<NX, NY>::NT;
+  constexpr int LS = PlaneCfg<NX, NY>::LS;
   constexpr int AX = nsplit_for(NX).n1, BX = nsplit_for(NX).n2;
   constexpr int AY = nsplit_for(NY).n1, BY = nsplit_for(NY).n2;
   extern __shared__ unsigned char smem_raw[];
   T *plane = reinterpret_cast<T *>(smem_raw);
   T *wx = plane + NY * LS;
   T *wy = wx + NX;
-  int *xa = reinterpret_cast<int *>(wy + NY);  // x -> active index or -1
+  int *xoff = reinterpret_cast<int *>(wy + NY);
   double *acc = reinterpret_cast<double *>(smem_raw + plane_rho_acc_off<NX, NY, T>());
-  const int la = g.nxa | 1;
   const int zp = blockIdx.x, grp = blockIdx.y;
-  for (int t = threadIdx.x; t < NX; t += NT) {
-    wx[t] = wx_g[t];
-    xa[t] = g.xa_of_x[t];
-  }
-  for (int t = threadIdx.x; t < NY; t += NT) wy[t] = wy_g[t];
-  for (int e = threadIdx.x; e < NX * NY; e += NT) acc[e] = 0.0;
-  const Lines cols{nullptr, 1, g.nxa};
+  for (int t = threadIdx.x; t < NX; t += blockDim.x) wx[t] = wx_g[t];
+  for (int t = threadIdx.x; t < NY; t += blockDim.x) wy[t] = wy_g[t];
+  for (int t = threadIdx.x; t < g.nxa; t += blockDim.x) xoff[t] = g.xa_list[t];
+  for (int e = threadIdx.x; e < NX * NY; e += blockDim.x) acc[e] = 0.0;
+  const Lines cols{xoff, 0, g.nxa};
   const Lines rows{nullptr, LS, NY};
   const int b0 = grp * bands_per_group, b1 = min(nbb, b0 + bands_per_group);
   for (int band = b0; band < b1; band++) {
     const T *Sz = S + ((size_t)band * n3 + zp) * g.ncol;
     __syncthreads();
-    for (int e = threadIdx.x; e < NY * la; e += NT) plane[e] = czero<T>();
+    for (int e = threadIdx.x; e < NY * LS; e += blockDim.x) plane[e] = czero<T>();
     __syncthreads();
-    for (int c = threadIdx.x; c < g.ncol; c += NT)
-      plane[g.col_y[c] * la + xa[g.col_x[c]]] = Sz[c];
+    for (int c = threadIdx.x; c < g.ncol; c += blockDim.x)
+      plane[g.col_y[c] * LS + g.col_x[c]] = Sz[c];
     __syncthreads();
-    inv_stepS<AY, BY>(plane, cols, la, wy);
+    inv_stepS<AY, BY>(plane, cols, LS, wy);
     __syncthreads();
-    inv_stepB<AY, BY>(plane, cols, la, wy);
+    inv_stepB<AY, BY>(plane, cols, LS, wy);
     __syncthreads();
-    x_inv_expand<NY, AX, BX, NT>(plane, la, LS, xa, wx);
+    inv_stepS<AX, BX>(plane, rows, 1, wx);
     __syncthreads();
     inv_stepB<AX, BX>(plane, rows, 1, wx);
     __syncthreads();
     const double w = wband[band];
-    for (int e = threadIdx.x; e < NX * NY; e += NT) {
+    for (int e = threadIdx.x; e < NX * NY; e += blockDim.x) {
       const int y = e / NX, x = e - y * NX;
       const T v = plane[y * LS + x];
       acc[e] += w * ((double)v.x * (double)v.x + (double)v.y * (double)v.y);
@@ -294,7 +292,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NT) k_plane_rho(
   }
   __syncthreads();
   double *pp = part + ((size_t)grp * n3 + zp) * NX * NY;
-  for (int e = threadIdx.x; e < NX * NY; e += NT) pp[e] = acc[e];
+  for (int e = threadIdx.x; e < NX * NY; e += blockDim.x) pp[e] = acc[e];
 }
 
 // ---- host-side launchers
