@@ -102,7 +102,9 @@ __global__ void k_fold_build(const int2 *__restrict__ pair, int groups, int ngw,
 // Tiles of (32 WM) x (16 WN) outputs, warps of 32 x 16.
 template <int WM, int WN>
 struct Ft {
-  static constexpr int BM = 32 * WM, BN = 16 * WN, BK = 16, STAGES = 3;
+  // two ring slots for the 64 x 32 tile: with three, shared memory held 3 of
+  // the 4 blocks per SM that registers allow
+  static constexpr int BM = 32 * WM, BN = 16 * WN, BK = 16, STAGES = WM * WN == 4 ? 2 : 3;
   static constexpr int THREADS = 32 * WM * WN;
   // padded so that the fragment loads of a half warp (8-byte B) or a quarter
   // warp (16-byte psi) hit distinct banks: 4 mod 16 doubles, 4 mod 8 complex

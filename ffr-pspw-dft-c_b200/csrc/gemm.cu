@@ -287,7 +287,9 @@ __global__ void k_zgemm_reduce_warp(int m, int n, int nsplit, const cx<R> *__res
 // tiles against 192 with 64-wide ones).
 template <int WM, int WN>
 struct Dm {
-  static constexpr int BM = 32 * WM, BN = 16 * WN, BK = 8, STAGES = 4;
+  // three ring slots for the tiles of 2 and 4 warps: with four, shared memory
+  // held 4 of the 8 (3 of the 4) blocks per SM that registers allow
+  static constexpr int BM = 32 * WM, BN = 16 * WN, BK = 8, STAGES = WM * WN <= 4 ? 3 : 4;
   static constexpr int THREADS = 32 * WM * WN;
   // [row][k] tiles: BK + 4 = 12 complex per row (12 = 4 mod 8): the fragment
   // loads of a quarter warp (rows g, g+1; k = t..t+3) cover 8 distinct
@@ -298,6 +300,10 @@ struct Dm {
   static constexpr int STAGE = A_ELEMS + B_ELEMS;  // complex elements per ring slot
   static constexpr size_t SMEM = sizeof(double2) * STAGE * STAGES;
   static constexpr int MIN_BLOCKS = 16 / (WM * WN);  // 2, 4 or 8 blocks of registers per SM
+  // blocks that shared memory lets an SM hold at once
+  static constexpr int RESIDENT = (int)(228 * 1024 / (SMEM + 1024)) < MIN_BLOCKS
+                                      ? (int)(228 * 1024 / (SMEM + 1024))
+                                      : MIN_BLOCKS;
 };
 
 // part or C over the block's K slice [blockIdx.z * kchunk, +kchunk)
@@ -443,7 +449,7 @@ static int launch_dmma(pspw_cell *c, bool conj, int m, int n, int k, double2 alp
   const int mt = (m + D::BM - 1) / D::BM, nt = (n + D::BN - 1) / D::BN;
   // K split over blocks when the output has fewer blocks than the SMs hold
   // (kZgemmUpperC: the tiles below the diagonal end at once and do not count)
-  const int target = D::MIN_BLOCKS * sm_count_now();
+  const int target = D::RESIDENT * sm_count_now();
   int tiles = mt * nt;
   if (tri == kZgemmUpperC)
     for (int i = 0; i < mt; i++)
