@@ -588,8 +588,6 @@ int swap_stick_order(pspw_cell *c) {
         (rc = gather_copy(c, P.d_pkga64, P.nproj > 0 ? P.nsp : 0, 4, &S.pkga64)) ||
         (rc = gather_copy(c, P.d_pkga32, P.nproj > 0 ? P.nsp : 0, 4, &S.pkga32)))
       return rc;
-    // (with the pair symmetry the filter's products run over pairs only)
-    if (!P.fold.ok && P.d_etp && S.eigr32 && (rc = nl_tc_build_tiles(c, S.eigr32, &S.etp, &S.etb))) return rc;
     S.built = true;
   }
   std::swap(B.d_sg_ig, S.sg_ig);

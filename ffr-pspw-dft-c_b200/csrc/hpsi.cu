@@ -772,11 +772,14 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
     timing_end(c, fam, e);
     c->kernel_launches++;
   };
-  // FP32 with one species: projector GEMMs on the tensor cores
+  // products over pairs (+G, -G) where the projectors have that symmetry; FP32
+  // on the tensor cores, where a caller with a scratch plan (no allocation)
+  // needs the operand tiles to be there already
+  const bool pairs = nproj > 0 && fold_usable(c, ngw);
   bool use_tc = false;
-  if constexpr (sizeof(R) == 4) use_tc = nproj > 0 && nl_tc_usable(c);
-  // products over pairs (+G, -G) where the projectors have that symmetry
-  const bool fold = (sizeof(R) == 8 || use_tc) && nproj > 0 && !plan && fold_usable(c, ngw);
+  if constexpr (sizeof(R) == 4)
+    use_tc = nproj > 0 && nl_tc_usable(c) && (!plan || nl_tc_have_tiles(c, pairs));
+  const bool fold = pairs && (use_tc || (sizeof(R) == 8 && !plan));
   float *tc_part = nullptr, *tc_wt = nullptr;
   int tc_split = 0;
   // The projection reads psi only: it runs on the cell's second stream,
@@ -865,7 +868,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
         tc_wt = static_cast<float *>(plan->wt);
         tc_split = plan->max_split;
       } else {
-        int rc = fold ? nl_tc_pair_tiles(c) : PSPW_OK;
+        int rc = nl_tc_ensure_tiles(c, fold);
         if (rc) return rc;
         if ((rc = nl_tc_reserve(c, ngw, nb, &tc_part, &tc_split, &tc_wt, fold))) return rc;
       }

@@ -1015,11 +1015,10 @@ int nl_tc_wait_check(pspw_cell *c, int complete) {
 bool nl_tc_usable(const pspw_cell *c) {
   static const bool off = std::getenv("PSPW_NL_SIMT") != nullptr;
   if (c->nl_path == PSPW_NL_SIMT || (off && c->nl_path != PSPW_NL_TENSOR_CORE)) return false;
-  // (in the filter's stick order a cell with pair symmetry has no other tiles)
-  return fits(c->proj) && ((c->proj.d_etp && c->proj.d_etb) || c->proj.fold.ok) && c->d_err;
+  return fits(c->proj) && c->d_err;
 }
 
-int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **etb) {
+static int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **etb) {
   Projectors &P = c->proj;
   if (!fits(P)) return PSPW_OK;
   const int ngw = c->basis.ngw;
@@ -1053,10 +1052,9 @@ int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **e
   return PSPW_OK;
 }
 
-int nl_tc_pair_tiles(pspw_cell *c) {
+static int nl_tc_pair_tiles(pspw_cell *c) {
   Projectors &P = c->proj;
   Fold &f = P.fold;
-  if (f.etp) return PSPW_OK;
   const int ngw = c->basis.ngw, n = 8 * f.groups;
   const std::vector<Group> gs = groups_of(P, ngw, true);
   const int nst = (n + kStepG - 1) / kStepG * (kStepG / 8), ngt = (n + 127) / 128;
@@ -1085,9 +1083,18 @@ int nl_tc_pair_tiles(pspw_cell *c) {
 }
 
 int nl_tc_prepare(pspw_cell *c) {
+  if (!fits(c->proj)) return PSPW_OK;
+  return nl_tc_ensure_tiles(c, c->proj.fold.ok);
+}
+
+bool nl_tc_have_tiles(const pspw_cell *c, bool fold) {
+  return fold ? c->proj.fold.etp != nullptr : c->proj.d_etp != nullptr;
+}
+
+int nl_tc_ensure_tiles(pspw_cell *c, bool fold) {
+  if (nl_tc_have_tiles(c, fold)) return PSPW_OK;
   Projectors &P = c->proj;
-  if (!fits(P) || P.d_etp) return PSPW_OK;
-  return nl_tc_build_tiles(c, P.d_eigr32, &P.d_etp, &P.d_etb);
+  return fold ? nl_tc_pair_tiles(c) : nl_tc_build_tiles(c, P.d_eigr32, &P.d_etp, &P.d_etb);
 }
 
 size_t nl_tc_wtile_bytes(const pspw_cell *c, int nb) {

@@ -10,15 +10,14 @@ namespace pspw {
 // kernels are selected.  The kernels run once per such species.
 bool nl_tc_usable(const pspw_cell *c);
 
-// Builds the EIGR operand tiles of a cell whose projectors fit the kernels
-// (no-op otherwise).  Called once at cell creation.
+// EIGR operand tiles of the cell's current G order, over pairs (fold; the
+// cell's fold must be ok) or over G.  A new cell gets those that its products
+// over the whole sphere use (nl_tc_prepare, no-op when the projectors do not
+// fit the kernels); the others, and the stick order's, are built when they
+// are first needed.
 int nl_tc_prepare(pspw_cell *c);
-// The same tiles from a given EIGR copy (FP32, [nat][ngw]) into new buffers.
-int nl_tc_build_tiles(pspw_cell *c, const float2 *eigr32, float **etp, float **etb);
-
-// The tiles over pairs (+G, -G) of the cell's current G order (its fold must
-// be ok), built on the first call of each order.
-int nl_tc_pair_tiles(pspw_cell *c);
+bool nl_tc_have_tiles(const pspw_cell *c, bool fold);
+int nl_tc_ensure_tiles(pspw_cell *c, bool fold);
 
 // Bytes of the projection operand tiles for nb bands.
 size_t nl_tc_wtile_bytes(const pspw_cell *c, int nb);
@@ -30,7 +29,7 @@ int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, f
 
 // Projections of nb bands (first ngw G) into the operand tiles `wt`:
 // W(a,lm,b) = WNL(lm) sum_G conj(EIGR(G,a)) PKG_A(lm,G) psi_b(G).
-// fold (in all three): over pairs, after nl_tc_pair_tiles.
+// fold (in all three): over pairs; after nl_tc_ensure_tiles.
 int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, float *part,
                   int max_split, float *wt, bool fold);
 
