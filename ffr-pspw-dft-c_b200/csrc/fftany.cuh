@@ -19,7 +19,8 @@
 // integers per element, and took primes as direct sums on a local-memory
 // array.  Block H*psi, before -> with these kernels: 50 x 64 x 45, 93 bands
 // FP32 383 -> 124 us; 74^3, 32 bands FP64 10.5 -> 0.58 ms; six cells of
-// 30..60 points per axis in one batch, FP32 2.23 -> 0.72 ms.
+// 30..60 points per axis in one batch, FP32 2.23 -> 0.72 ms.  Per point of a
+// plane 6.9 ps (50 x 64, FP32) against 4.9 ps of the compiled 64 x 64.
 //
 // Primes above 13 hold the item's (p - 1) / 2 symmetric pairs in registers
 // and loop over the output pairs, with the cosines and sines broadcast from
@@ -499,6 +500,17 @@ int any_plane(const Basis &B, const FastGeo &g, cudaStream_t st, int nbb, const 
   constexpr bool f32 = sizeof(R) == 4;
   return with_class<0>(plane_class(p), [&](auto cls) -> int {
     constexpr int CLS = decltype(cls)::value;
+    if constexpr (CLS == 0) {
+      if (B.n1 * B.n2 < 6000) {
+        // blocks of 256 threads held to the registers of five (FP32: 63 -> 48)
+        // or three (FP64: 118 -> 80) per SM; shared memory leaves room for
+        // eight and four (six FP32 cells in a batch 683 -> 631 us)
+        auto k = k_plane_any<CLS, 256, f32 ? 5 : 3, T, R>;
+        if (const int rc = smem_allow_max(k)) return rc;
+        k<<<grid, 256, sm, st>>>(g, p, B.n3, wx, wy, vperm, S);
+        return PSPW_OK;
+      }
+    }
     constexpr int NT = CLS < 2 ? 512 : kPrimeThreads;
     constexpr int MB = (f32 && CLS == 0) || CLS == 2 ? 2 : 1;
     auto k = k_plane_any<CLS, NT, MB, T, R>;
