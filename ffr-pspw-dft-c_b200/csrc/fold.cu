@@ -99,7 +99,7 @@ __global__ void k_fold_build(const int2 *__restrict__ pair, int groups, int ngw,
   b[8] = o ? c : s;
 }
 
-// Tiles of (32 WM) x (16 WN) outputs, warps of 32 x 16.
+// Tiles of (32 WM) x (16 WN) outputs, warps of 32 x 16; WM 1 or 2, WN 1 to 4.
 template <int WM, int WN>
 struct Ft {
   // two ring slots for the 64 x 32 tile: with three, shared memory held 3 of
@@ -117,6 +117,10 @@ struct Ft {
   static constexpr size_t Q_SLOT = sizeof(double) * Q_A + sizeof(double2) * Q_X;
   static constexpr size_t P_SMEM = P_SLOT * STAGES, Q_SMEM = Q_SLOT * STAGES;
   static constexpr int MIN_BLOCKS = 16 / (WM * WN) > 8 ? 8 : 16 / (WM * WN);
+  // blocks that shared memory lets an SM hold at once
+  static constexpr int RESIDENT = (int)(228 * 1024 / (P_SMEM + 1024)) < MIN_BLOCKS
+                                      ? (int)(228 * 1024 / (P_SMEM + 1024))
+                                      : MIN_BLOCKS;
 };
 
 // part or wp over groups [blockIdx.z * gchunk, +gchunk): acc(p, b)
@@ -481,14 +485,16 @@ int ensure_b64(pspw_cell *c) {
   return PSPW_OK;
 }
 
-// Slices of the groups for `tiles` output tiles: the count whose last wave of
-// `target` resident blocks is fullest (Si216, 112 tiles of 64 x 64: two slices
-// fill 76 % of the one wave they need and took 7.8 ms), among those that leave
-// 16 groups or more per slice; more slices only when they gain 2 %.
-int fold_slices(int tiles, int target, int most) {
-  int best = 1;
-  double best_fill = 0.0;
-  for (int n = 1; n <= std::min(most, std::max(16, 2 * target / tiles)); n++) {
+// Slices of the groups for `tiles` output tiles: what one wave of `target`
+// resident blocks holds, or more when a fuller last wave gains 2 % (Si216, 112
+// tiles of 64 x 64: two slices fill 76 % of their wave and took 7.8 ms, 13 fill
+// 98 % and take 5.9), in slices of four groups or more and at most 96 (the
+// partial sums are written and read once more).
+int fold_slices(int tiles, int target, int groups) {
+  const int most = std::max(1, std::min(96, groups / 4));
+  int best = std::max(1, std::min(most, target / tiles));
+  double best_fill = std::min(1.0, (double)tiles * best / target);
+  for (int n = best + 1; n <= std::min(most, 16); n++) {
     const double waves = (double)tiles * n / target;
     const double fill = waves / std::ceil(waves);
     if (fill > best_fill + 0.02) {
@@ -505,8 +511,8 @@ int launch_proj(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, c
   const Projectors &P = c->proj;
   const Fold &f = P.fold;
   const int mt = (P.nproj + F::BM - 1) / F::BM, nt = (nb + F::BN - 1) / F::BN;
-  const int target = F::MIN_BLOCKS * sm_count_now();
-  int nsplit = fold_slices(mt * nt, target, (f.groups + 15) / 16);
+  const int target = F::RESIDENT * sm_count_now();
+  int nsplit = fold_slices(mt * nt, target, f.groups);
   const int gchunk = (f.groups + nsplit - 1) / nsplit;
   nsplit = (f.groups + gchunk - 1) / gchunk;
   double2 *part = nullptr;
@@ -676,11 +682,23 @@ int fold_project64(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp
     PSPW_CUDA(cudaGetLastError());
     return PSPW_OK;
   }
+  // 32-row tiles where 64-row ones would pad the projectors by more than a
+  // tenth (32 projectors: half the tile)
+  const int r64 = (P.nproj + 63) / 64 * 64, r32 = (P.nproj + 31) / 32 * 32;
+  const bool narrow = 10 * r64 > 11 * r32;
   switch (tile_bands(nb)) {
-    case 64: return launch_proj<2, 4>(c, psi, ld, nb, wp, w);
-    case 48: return launch_proj<2, 3>(c, psi, ld, nb, wp, w);
-    case 32: return launch_proj<2, 2>(c, psi, ld, nb, wp, w);
-    default: return launch_proj<2, 1>(c, psi, ld, nb, wp, w);
+    case 64:
+      return narrow ? launch_proj<1, 4>(c, psi, ld, nb, wp, w)
+                    : launch_proj<2, 4>(c, psi, ld, nb, wp, w);
+    case 48:
+      return narrow ? launch_proj<1, 3>(c, psi, ld, nb, wp, w)
+                    : launch_proj<2, 3>(c, psi, ld, nb, wp, w);
+    case 32:
+      return narrow ? launch_proj<1, 2>(c, psi, ld, nb, wp, w)
+                    : launch_proj<2, 2>(c, psi, ld, nb, wp, w);
+    default:
+      return narrow ? launch_proj<1, 1>(c, psi, ld, nb, wp, w)
+                    : launch_proj<2, 1>(c, psi, ld, nb, wp, w);
   }
 }
 
@@ -695,11 +713,22 @@ int fold_backproject64(pspw_cell *c, const double2 *wp, int nb, double2 *out, in
     PSPW_CUDA(cudaGetLastError());
     return PSPW_OK;
   }
-  switch (tile_bands(nb)) {
-    case 64: return launch_back<2, 4>(c, wp, nb, out, ldo, alpha);
-    case 48: return launch_back<2, 3>(c, wp, nb, out, ldo, alpha);
-    case 32: return launch_back<2, 2>(c, wp, nb, out, ldo, alpha);
-    default: return launch_back<2, 1>(c, wp, nb, out, ldo, alpha);
+  // 32-row tiles (two groups) where 64-row ones would leave SMs without a block
+  const int bands = tile_bands(nb);
+  const bool few = (f.groups + 3) / 4 * ((nb + bands - 1) / bands) < sm_count_now();
+  switch (bands) {
+    case 64:
+      return few ? launch_back<1, 4>(c, wp, nb, out, ldo, alpha)
+                 : launch_back<2, 4>(c, wp, nb, out, ldo, alpha);
+    case 48:
+      return few ? launch_back<1, 3>(c, wp, nb, out, ldo, alpha)
+                 : launch_back<2, 3>(c, wp, nb, out, ldo, alpha);
+    case 32:
+      return few ? launch_back<1, 2>(c, wp, nb, out, ldo, alpha)
+                 : launch_back<2, 2>(c, wp, nb, out, ldo, alpha);
+    default:
+      return few ? launch_back<1, 1>(c, wp, nb, out, ldo, alpha)
+                 : launch_back<2, 1>(c, wp, nb, out, ldo, alpha);
   }
 }
 
