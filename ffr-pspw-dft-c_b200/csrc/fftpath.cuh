@@ -169,14 +169,16 @@ constexpr size_t plane_smem() {
   return sizeof(T) * ((size_t)NY * PlaneCfg<NX, NY>::LS + NX + NY) + sizeof(int) * NX;
 }
 
-// FP64 planes of 256 threads whose shared memory leaves room for three blocks
-// per SM are held to the registers of three (64 x 64: 88 -> 80)
+// FP64 planes of 60 and 64 points per axis, which take 100 and 88 registers
+// (two blocks per SM), are held to the registers of three, for which shared
+// memory has room (150 bands: 256 -> 232 and 246 -> 225 us).  All others leave
+// it to the compiler (0): a bound they do not need costs them 5 to 10 %.
 template <int NX, int NY, typename T>
 constexpr int plane_min_blocks() {
-  return sizeof(T) == 16 && PlaneCfg<NX, NY>::NT == 256 &&
+  return sizeof(T) == 16 && PlaneCfg<NX, NY>::NT == 256 && NX >= 60 &&
                  3 * (plane_smem<NX, NY, T>() + 1024) <= 228 * 1024
              ? 3
-             : 1;
+             : 0;
 }
 
 // One z-plane of one band.  The y transforms and the stick scatter/gather
