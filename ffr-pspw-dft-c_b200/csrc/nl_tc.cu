@@ -74,7 +74,7 @@ constexpr int kTileBytes128 = 128 * kBK * 4;            // 128 rows x BK fp32
 constexpr uint32_t kLBO = 128, kSBO = (kBK / 4) * 128;  // core-matrix strides
 constexpr int kNTP = 4;                                 // operand slots, projection
 constexpr int kNTB = 2;                                 // operand slots, back-projection
-constexpr int kNR = 6;                                  // raw slots, projection
+constexpr int kNR = 6;                                  // raw slots, projection (at most)
 constexpr int kRowWarps = 8;                            // row / epilogue warps
 constexpr int kRowThreads = 32 * kRowWarps;
 constexpr int kThreads = kRowThreads + 64;              // + producer + MMA warps
@@ -169,6 +169,11 @@ constexpr int kStepG = 16;  // G per projection step
 // and bit lm of `odd` marks the odd form factors.
 __host__ __device__ constexpr int raw_row(bool fold) { return (fold ? 2 : 1) * (kStepG + 1); }
 
+// Raw slots in flight.  With one projector per atom a tile touches 65 bands and
+// a slot of pairs takes 18 KB: six of them beside the two EIGR slots of 241 to
+// 256 atoms (131 KB) would be 239 KB, more than a block can have.
+__host__ __device__ constexpr int raw_slots(int L, bool fold) { return fold && L == 1 ? 5 : kNR; }
+
 template <int L, bool FOLD>
 __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict__ psi, int ld,
                                                       int ngw, int nb,
@@ -184,6 +189,9 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
   constexpr int kMinus = kStepG + 1;      // FOLD: where the -G values start
   constexpr int raw_psi = round16(nbr_max * prow * 8);
   constexpr int raw_bytes = raw_psi + kStepG * 16;
+  constexpr int nr = raw_slots(L, FOLD);
+  // 256 atoms (the most that nl_tc_usable admits) have the largest tiles
+  static_assert(proj_slots(256) * 2 * 256 * 128 + nr * raw_bytes + sizeof(Sync) <= 227 * 1024);
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ Sync sy;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -198,7 +206,7 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
   unsigned char *raw0 = sm + nts * 2 * ebytes;
   const uint32_t acol = tmem_cols(npad);
   const uint32_t ncols = tmem_cols(acol + 64 * nts);
-  open_block(sy, ncols, nts, kRowWarps + 1, kNR);
+  open_block(sy, ncols, nts, kRowWarps + 1, nr);
 
   if (warp < kRowWarps) {
     // ---- A' rows
@@ -210,8 +218,8 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
     const int lm = (m % per) >> 1, p = m & 1;
     const bool is_odd = FOLD && ((odd >> lm) & 1);
     for (int k = 0; k < nsteps; k++) {
-      const int rs = k % kNR, ts = k % nts;
-      if (!tc::mbar_wait_abort(&sy.rfull[rs], (k / kNR) & 1, &sy.abort)) break;
+      const int rs = k % nr, ts = k % nts;
+      if (!tc::mbar_wait_abort(&sy.rfull[rs], (k / nr) & 1, &sy.abort)) break;
       if (k >= nts && !tc::mbar_wait_abort(&sy.empty[ts], ((k / nts) - 1) & 1, &sy.abort)) break;
       tc::fence_after_sync();
       const unsigned char *r = raw0 + rs * raw_bytes;
@@ -277,10 +285,10 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
     };
     int2 next = pair_at(0);
     for (int k = 0; k < nsteps; k++) {
-      const int rs = k % kNR;
+      const int rs = k % nr;
       const int2 pr = next;
       next = pair_at(k + 1);
-      if (k >= kNR && !tc::mbar_wait_abort(&sy.rempty[rs], ((k / kNR) - 1) & 1, &sy.abort))
+      if (k >= nr && !tc::mbar_wait_abort(&sy.rempty[rs], ((k / nr) - 1) & 1, &sy.abort))
         break;
       unsigned char *r = raw0 + rs * raw_bytes;
       float2 *rp = reinterpret_cast<float2 *>(r);
@@ -905,7 +913,8 @@ int proj_tmem_cols(const Shape &s) {
 int proj_smem(const Shape &s, bool fold) {
   const int nbr_max = 127 / s.per + 2;
   const int raw = round16(nbr_max * raw_row(fold) * 8) + kStepG * 16;
-  return block_smem(proj_slots(s.npad) * 2 * s.npad * 128 + kNR * raw, proj_tmem_cols(s));
+  return block_smem(proj_slots(s.npad) * 2 * s.npad * 128 + raw_slots(s.L, fold) * raw,
+                    proj_tmem_cols(s));
 }
 
 int backpair_smem(const Shape &s) {
