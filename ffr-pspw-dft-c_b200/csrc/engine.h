@@ -74,6 +74,7 @@ struct Basis {
 struct Fold {
   bool ok = false;
   int groups = 0;           // groups of 8 pairs (the last padded)
+  std::vector<int> first;   // x of each group's first pair, ascending (host)
   int2 *d_pair = nullptr;   // [8 * groups] G indices of the pair; y < 0: G = 0, x < 0: padding
   double *d_b64 = nullptr;  // [16 * groups x nproj] column-major, built on first use
   // FP32 operand tiles of the tensor-core GEMMs over pairs (nl_tc.cu), built on

@@ -17,8 +17,10 @@
 // w'_p = W_p times the real sums, for both parities.
 //
 // The symmetry is checked bit for bit for every atom, projector and G when
-// the cell is created (any caller's arrays come in); cells without it, and
-// products over fewer G than the sphere, keep the complex GEMM of gemm.cu.
+// the cell is created (any caller's arrays come in); cells without it keep the
+// complex GEMM of gemm.cu.  A call over the first ngw G only treats the others
+// as absent (psi = 0, nothing written) and stops at the last pair that has one:
+// at worst (no G's partner among them) that is the work of the complex GEMM.
 //
 // Kernels: DMMA tiles as in gemm.cu (warps of 32 x 16 outputs, cp.async
 // ring).  A K step of the projection is one group of 8 pairs = 16 real rows:
@@ -49,6 +51,12 @@ namespace pspw {
 namespace {
 
 constexpr int kGroup = 8;  // pairs per group; 16 rows of B
+
+// The pair as a call over the first ngw G sees it: -1 for a G that is not
+// among them.  (x < y in every pair, so x is missing only where both are.)
+__device__ __forceinline__ int2 below(int2 p, int ngw) {
+  return make_int2(p.x < ngw ? p.x : -1, p.y < ngw ? p.y : -1);
+}
 
 // flags: [0] EIGR symmetric, [1 + 2 (4 s + lm)] even holds, [.. + 1] odd holds
 __global__ void k_fold_check(const int2 *__restrict__ pair, int npair, int ngw, int nat, int nsp,
@@ -123,18 +131,18 @@ struct Ft {
                                       : MIN_BLOCKS;
 };
 
-// part or wp over groups [blockIdx.z * gchunk, +gchunk): acc(p, b)
+// part or wp over groups [blockIdx.z * gchunk, +gchunk) below `used`: acc(p, b)
 template <int WM, int WN>
 __global__ void __launch_bounds__(Ft<WM, WN>::THREADS, Ft<WM, WN>::MIN_BLOCKS)
-    k_fold_proj(const double *__restrict__ B, const int2 *__restrict__ pair, int groups,
-                int nproj, const double2 *__restrict__ psi, int ld, int nb, int gchunk,
+    k_fold_proj(const double *__restrict__ B, const int2 *__restrict__ pair, int groups, int used,
+                int ngw, int nproj, const double2 *__restrict__ psi, int ld, int nb, int gchunk,
                 const double *__restrict__ w, const unsigned char *__restrict__ odd,
                 double2 *__restrict__ wp, double2 *__restrict__ part) {
   using F = Ft<WM, WN>;
   constexpr int BM = F::BM, BN = F::BN, STAGES = F::STAGES, THREADS = F::THREADS;
   extern __shared__ __align__(16) unsigned char raw[];
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int g0 = blockIdx.z * gchunk, g1 = min(groups, g0 + gchunk);
+  const int g0 = blockIdx.z * gchunk, g1 = min(used, g0 + gchunk);
   const int nst = g1 - g0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = (warp % WM) * 32, wn = (warp / WM) * 16;
@@ -150,7 +158,8 @@ __global__ void __launch_bounds__(Ft<WM, WN>::THREADS, Ft<WM, WN>::MIN_BLOCKS)
   auto index = [&](int st) {
     if (st >= nst) return -1;
     const int2 p = pair[(g0 + st) * kGroup + (kk & 7)];
-    return kk < 8 ? p.x : p.y;
+    const int g = kk < 8 ? p.x : p.y;
+    return g < ngw ? g : -1;
   };
   auto load = [&](int st, int slot, int ig) {
     double *As = slotA(slot);
@@ -261,8 +270,8 @@ __global__ void k_fold_reduce(const double2 *__restrict__ part, int nsplit, int 
 // rows of groups [blockIdx.x * BM / 16, ...) x bands: out(+-G) += alpha (A +- i Q)
 template <int WM, int WN>
 __global__ void __launch_bounds__(Ft<WM, WN>::THREADS, Ft<WM, WN>::MIN_BLOCKS)
-    k_fold_back(const double *__restrict__ B, const int2 *__restrict__ pair, int groups,
-                int nproj, const double2 *__restrict__ wp, int nb, double2 *out, int ldo,
+    k_fold_back(const double *__restrict__ B, const int2 *__restrict__ pair, int groups, int used,
+                int ngw, int nproj, const double2 *__restrict__ wp, int nb, double2 *out, int ldo,
                 double alpha) {
   using F = Ft<WM, WN>;
   constexpr int BM = F::BM, BN = F::BN, BK = F::BK, STAGES = F::STAGES, THREADS = F::THREADS;
@@ -337,8 +346,8 @@ __global__ void __launch_bounds__(Ft<WM, WN>::THREADS, Ft<WM, WN>::MIN_BLOCKS)
 #pragma unroll
   for (int i = 0; i < 2; i++) {
     const int grp = (m0 + wm + i * 16) >> 4;
-    if (grp >= groups) continue;
-    const int2 pr = pair[grp * kGroup + g];
+    if (grp >= used) continue;
+    const int2 pr = below(pair[grp * kGroup + g], ngw);
     if (pr.x < 0) continue;
 #pragma unroll
     for (int j = 0; j < 2; j++)
@@ -365,20 +374,20 @@ constexpr int kVP = 4;  // projectors per block of the matrix-vector projection
 
 // part[slice][p]: blocks of 4 columns over a slice of the pairs
 __global__ void __launch_bounds__(256)
-    k_fold_projv(const double *__restrict__ B, const int2 *__restrict__ pair, int groups,
-                 int nproj, const double2 *__restrict__ psi, int gchunk,
+    k_fold_projv(const double *__restrict__ B, const int2 *__restrict__ pair, int groups, int used,
+                 int ngw, int nproj, const double2 *__restrict__ psi, int gchunk,
                  const double *__restrict__ w, const unsigned char *__restrict__ odd,
                  double2 *__restrict__ wp, double2 *__restrict__ part) {
   __shared__ double2 red[8][kVP];
   const size_t rows = 16 * (size_t)groups;
   const int p0 = blockIdx.x * kVP;
-  const int j0 = blockIdx.y * gchunk * kGroup, j1 = min(groups, (blockIdx.y + 1) * gchunk) * kGroup;
+  const int j0 = blockIdx.y * gchunk * kGroup, j1 = min(used, (blockIdx.y + 1) * gchunk) * kGroup;
   double2 s[kVP];
 #pragma unroll
   for (int q = 0; q < kVP; q++) s[q] = make_double2(0.0, 0.0);
 #pragma unroll 2
   for (int j = j0 + threadIdx.x; j < j1; j += 256) {
-    const int2 pr = pair[j];
+    const int2 pr = below(pair[j], ngw);
     const double2 zero = make_double2(0.0, 0.0);
     const double2 x = pr.x >= 0 ? psi[pr.x] : zero, y = pr.y >= 0 ? psi[pr.y] : zero;
     const double ur = x.x + y.x, ui = x.y + y.y, vr = x.y - y.y, vi = y.x - x.x;
@@ -422,13 +431,13 @@ __global__ void __launch_bounds__(256)
 // 32 pairs per block, 8 warps over the projectors (p = warp, warp + 8, ...),
 // partial sums added in warp order
 __global__ void __launch_bounds__(256)
-    k_fold_backv(const double *__restrict__ B, const int2 *__restrict__ pair, int groups,
-                 int nproj, const double2 *__restrict__ wp, double2 *out, double alpha) {
+    k_fold_backv(const double *__restrict__ B, const int2 *__restrict__ pair, int groups, int used,
+                 int ngw, int nproj, const double2 *__restrict__ wp, double2 *out, double alpha) {
   __shared__ double4 red[8][32];
   const size_t rows = 16 * (size_t)groups;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
-  const bool on = j < groups * kGroup;
+  const bool on = j < used * kGroup;
   double ax = 0.0, ay = 0.0, qx = 0.0, qy = 0.0;
   if (on) {
     const double *b = B + (size_t)(j >> 3) * 16 + (j & 7);
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(256)
   red[warp][lane] = make_double4(ax, ay, qx, qy);
   __syncthreads();
   if (warp != 0 || !on) return;
-  const int2 pr = pair[j];
+  const int2 pr = below(pair[j], ngw);
   if (pr.x < 0) return;
   const double2 h = out[pr.x], l = pr.y >= 0 ? out[pr.y] : make_double2(0.0, 0.0);
 #pragma unroll
@@ -506,15 +515,16 @@ int fold_slices(int tiles, int target, int groups) {
 }
 
 template <int WM, int WN>
-int launch_proj(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, const double *w) {
+int launch_proj(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, double2 *wp,
+                const double *w) {
   using F = Ft<WM, WN>;
   const Projectors &P = c->proj;
   const Fold &f = P.fold;
   const int mt = (P.nproj + F::BM - 1) / F::BM, nt = (nb + F::BN - 1) / F::BN;
-  const int target = F::RESIDENT * sm_count_now();
-  int nsplit = fold_slices(mt * nt, target, f.groups);
-  const int gchunk = (f.groups + nsplit - 1) / nsplit;
-  nsplit = (f.groups + gchunk - 1) / gchunk;
+  const int target = F::RESIDENT * sm_count_now(), used = fold_groups(f, ngw);
+  int nsplit = fold_slices(mt * nt, target, used);
+  const int gchunk = (used + nsplit - 1) / nsplit;
+  nsplit = (used + gchunk - 1) / gchunk;
   double2 *part = nullptr;
   if (nsplit > 1) {
     const int rc = ws_reserve(c, kWsProjPart, sizeof(double2) * (size_t)nsplit * nb * P.nproj,
@@ -524,7 +534,7 @@ int launch_proj(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, c
   auto kern = k_fold_proj<WM, WN>;
   if (const int rc = smem_allow_max(kern)) return rc;
   kern<<<dim3(mt, nt, nsplit), F::THREADS, F::P_SMEM, c->stream>>>(
-      f.d_b64, f.d_pair, f.groups, P.nproj, psi, ld, nb, gchunk, w, P.d_odd, wp, part);
+      f.d_b64, f.d_pair, f.groups, used, ngw, P.nproj, psi, ld, nb, gchunk, w, P.d_odd, wp, part);
   c->kernel_launches++;
   if (nsplit > 1) {
     // small blocks: few outputs with many slices spread over more SMs
@@ -537,15 +547,17 @@ int launch_proj(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, c
 }
 
 template <int WM, int WN>
-int launch_back(pspw_cell *c, const double2 *wp, int nb, double2 *out, int ldo, double alpha) {
+int launch_back(pspw_cell *c, const double2 *wp, int ngw, int nb, double2 *out, int ldo,
+                double alpha) {
   using F = Ft<WM, WN>;
   const Projectors &P = c->proj;
   const Fold &f = P.fold;
   auto kern = k_fold_back<WM, WN>;
   if (const int rc = smem_allow_max(kern)) return rc;
-  const dim3 grid((16 * f.groups + F::BM - 1) / F::BM, (nb + F::BN - 1) / F::BN);
-  kern<<<grid, F::THREADS, F::Q_SMEM, c->stream>>>(f.d_b64, f.d_pair, f.groups, P.nproj, wp, nb,
-                                                   out, ldo, alpha);
+  const int used = fold_groups(f, ngw);
+  const dim3 grid((16 * used + F::BM - 1) / F::BM, (nb + F::BN - 1) / F::BN);
+  kern<<<grid, F::THREADS, F::Q_SMEM, c->stream>>>(f.d_b64, f.d_pair, f.groups, used, ngw, P.nproj,
+                                                   wp, nb, out, ldo, alpha);
   c->kernel_launches++;
   PSPW_CUDA(cudaGetLastError());
   return PSPW_OK;
@@ -603,6 +615,10 @@ int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, c
   stick_pairs.resize((size_t)groups * kGroup, make_int2(-1, -1));
   Fold &f = P.fold, &fs = c->stick.fold;
   f.groups = fs.groups = groups;
+  for (int g = 0; g < groups; g++) {  // (the last group has a pair too)
+    f.first.push_back(nat_pairs[(size_t)g * kGroup].x);
+    fs.first.push_back(stick_pairs[(size_t)g * kGroup].x);
+  }
   std::vector<int> flags(1 + 8 * (size_t)P.nsp, 1);
   // one allocation: both pair tables, the check's flags, the odd marks
   const size_t np = nat_pairs.size(), bytes = sizeof(int2) * np;
@@ -649,7 +665,12 @@ int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, c
   return run();
 }
 
-int fold_project64(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, bool plain) {
+int fold_groups(const Fold &f, int ngw) {
+  return (int)(std::lower_bound(f.first.begin(), f.first.end(), ngw) - f.first.begin());
+}
+
+int fold_project64(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, double2 *wp,
+                   bool plain) {
   int rc = ensure_b64(c);
   if (rc) return rc;
   const Projectors &P = c->proj;
@@ -661,18 +682,19 @@ int fold_project64(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp
     // reduction launch: such a call is bound by its launches (Si8, 369 groups:
     // a call of 21 us with a reduction, 19 us without)
     const int pt = (P.nproj + kVP - 1) / kVP;
-    int nsplit = f.groups <= 512 ? 1
-                                 : std::max(1, std::min((f.groups + 63) / 64,
-                                                        4 * sm_count_now() / pt));
-    const int gchunk = (f.groups + nsplit - 1) / nsplit;
-    nsplit = (f.groups + gchunk - 1) / gchunk;
+    const int used = fold_groups(f, ngw);
+    int nsplit = used <= 512 ? 1
+                             : std::max(1, std::min((used + 63) / 64, 4 * sm_count_now() / pt));
+    const int gchunk = (used + nsplit - 1) / nsplit;
+    nsplit = (used + gchunk - 1) / gchunk;
     double2 *part = nullptr;
     if (nsplit > 1) {
       rc = ws_reserve(c, kWsProjPart, sizeof(double2) * (size_t)nsplit * P.nproj, (void **)&part);
       if (rc) return rc;
     }
-    k_fold_projv<<<dim3(pt, nsplit), 256, 0, c->stream>>>(f.d_b64, f.d_pair, f.groups, P.nproj,
-                                                          psi, gchunk, w, P.d_odd, wp, part);
+    k_fold_projv<<<dim3(pt, nsplit), 256, 0, c->stream>>>(f.d_b64, f.d_pair, f.groups, used, ngw,
+                                                          P.nproj, psi, gchunk, w, P.d_odd, wp,
+                                                          part);
     c->kernel_launches++;
     if (nsplit > 1) {
       k_fold_reduce<<<(P.nproj + 127) / 128, 128, 0, c->stream>>>(part, nsplit, 1, P.nproj, w,
@@ -688,47 +710,48 @@ int fold_project64(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp
   const bool narrow = 10 * r64 > 11 * r32;
   switch (tile_bands(nb)) {
     case 64:
-      return narrow ? launch_proj<1, 4>(c, psi, ld, nb, wp, w)
-                    : launch_proj<2, 4>(c, psi, ld, nb, wp, w);
+      return narrow ? launch_proj<1, 4>(c, psi, ld, ngw, nb, wp, w)
+                    : launch_proj<2, 4>(c, psi, ld, ngw, nb, wp, w);
     case 48:
-      return narrow ? launch_proj<1, 3>(c, psi, ld, nb, wp, w)
-                    : launch_proj<2, 3>(c, psi, ld, nb, wp, w);
+      return narrow ? launch_proj<1, 3>(c, psi, ld, ngw, nb, wp, w)
+                    : launch_proj<2, 3>(c, psi, ld, ngw, nb, wp, w);
     case 32:
-      return narrow ? launch_proj<1, 2>(c, psi, ld, nb, wp, w)
-                    : launch_proj<2, 2>(c, psi, ld, nb, wp, w);
+      return narrow ? launch_proj<1, 2>(c, psi, ld, ngw, nb, wp, w)
+                    : launch_proj<2, 2>(c, psi, ld, ngw, nb, wp, w);
     default:
-      return narrow ? launch_proj<1, 1>(c, psi, ld, nb, wp, w)
-                    : launch_proj<2, 1>(c, psi, ld, nb, wp, w);
+      return narrow ? launch_proj<1, 1>(c, psi, ld, ngw, nb, wp, w)
+                    : launch_proj<2, 1>(c, psi, ld, ngw, nb, wp, w);
   }
 }
 
-int fold_backproject64(pspw_cell *c, const double2 *wp, int nb, double2 *out, int ldo,
+int fold_backproject64(pspw_cell *c, const double2 *wp, int ngw, int nb, double2 *out, int ldo,
                        double alpha) {
   const Projectors &P = c->proj;
   const Fold &f = P.fold;
+  const int used = fold_groups(f, ngw);
   if (nb == 1) {
-    k_fold_backv<<<(f.groups * kGroup + 31) / 32, 256, 0, c->stream>>>(
-        f.d_b64, f.d_pair, f.groups, P.nproj, wp, out, alpha);
+    k_fold_backv<<<(used * kGroup + 31) / 32, 256, 0, c->stream>>>(
+        f.d_b64, f.d_pair, f.groups, used, ngw, P.nproj, wp, out, alpha);
     c->kernel_launches++;
     PSPW_CUDA(cudaGetLastError());
     return PSPW_OK;
   }
   // 32-row tiles (two groups) where 64-row ones would leave SMs without a block
   const int bands = tile_bands(nb);
-  const bool few = (f.groups + 3) / 4 * ((nb + bands - 1) / bands) < sm_count_now();
+  const bool few = (used + 3) / 4 * ((nb + bands - 1) / bands) < sm_count_now();
   switch (bands) {
     case 64:
-      return few ? launch_back<1, 4>(c, wp, nb, out, ldo, alpha)
-                 : launch_back<2, 4>(c, wp, nb, out, ldo, alpha);
+      return few ? launch_back<1, 4>(c, wp, ngw, nb, out, ldo, alpha)
+                 : launch_back<2, 4>(c, wp, ngw, nb, out, ldo, alpha);
     case 48:
-      return few ? launch_back<1, 3>(c, wp, nb, out, ldo, alpha)
-                 : launch_back<2, 3>(c, wp, nb, out, ldo, alpha);
+      return few ? launch_back<1, 3>(c, wp, ngw, nb, out, ldo, alpha)
+                 : launch_back<2, 3>(c, wp, ngw, nb, out, ldo, alpha);
     case 32:
-      return few ? launch_back<1, 2>(c, wp, nb, out, ldo, alpha)
-                 : launch_back<2, 2>(c, wp, nb, out, ldo, alpha);
+      return few ? launch_back<1, 2>(c, wp, ngw, nb, out, ldo, alpha)
+                 : launch_back<2, 2>(c, wp, ngw, nb, out, ldo, alpha);
     default:
-      return few ? launch_back<1, 1>(c, wp, nb, out, ldo, alpha)
-                 : launch_back<2, 1>(c, wp, nb, out, ldo, alpha);
+      return few ? launch_back<1, 1>(c, wp, ngw, nb, out, ldo, alpha)
+                 : launch_back<2, 1>(c, wp, ngw, nb, out, ldo, alpha);
   }
 }
 

@@ -12,18 +12,20 @@ namespace pspw {
 // creation, after the projector arrays; leaves fold.ok false otherwise.
 int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, const int *order);
 
-// True when a product over the first ngw G may run over pairs.
-inline bool fold_usable(const pspw_cell *c, int ngw) {
-  return c->proj.fold.ok && ngw == c->basis.ngw;
-}
+// Groups that hold a pair with one of the first ngw G (pairs are in ascending
+// order of their first G).
+int fold_groups(const Fold &f, int ngw);
 
 // wp(p, b) = W_p acc(p, b) for the back-projection, acc the real-matrix sums:
 // the projections are acc for even p and i acc for odd p.  With `plain`, the
-// unweighted projections themselves.  wp: nproj x nb, column-major.
-int fold_project64(pspw_cell *c, const double2 *psi, int ld, int nb, double2 *wp, bool plain);
+// unweighted projections themselves.  wp: nproj x nb, column-major.  The sums
+// are over the first ngw G (in the stick order: all of them).
+int fold_project64(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, double2 *wp,
+                   bool plain);
 
-// out(:, b) += alpha sum_p beta_p (projections of p, b), from fold_project64's wp
-int fold_backproject64(pspw_cell *c, const double2 *wp, int nb, double2 *out, int ldo,
+// out(G, b) += alpha sum_p beta_p(G) (projections of p, b) for the first ngw G,
+// from fold_project64's wp
+int fold_backproject64(pspw_cell *c, const double2 *wp, int ngw, int nb, double2 *out, int ldo,
                        double alpha);
 
 }  // namespace pspw

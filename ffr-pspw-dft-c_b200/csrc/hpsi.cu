@@ -31,9 +31,9 @@
 // back-projection, whose epilogue also applies out = a*(H psi) + b*psi + g*x,
 // the update of the Chebyshev three-term recurrence (chebyfilt.cpp:36-59).
 // FP64: products over pairs (+G, -G) with a real projector matrix on the FP64
-// tensor-core instruction (fold.cu); without that symmetry, or over fewer G,
-// beta stored once per cell (NGW x nproj) and both products on the complex
-// GEMM (gemm.cu).  The allocation-free entry point keeps the SIMT kernels.
+// tensor-core instruction (fold.cu); without that symmetry, beta stored once
+// per cell (NGW x nproj) and both products on the complex GEMM (gemm.cu).  The
+// allocation-free entry point keeps the SIMT kernels.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -773,12 +773,12 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
     c->kernel_launches++;
   };
   // products over pairs (+G, -G) where the projectors have that symmetry; FP32
-  // on the tensor cores, where a caller with a scratch plan (no allocation)
-  // needs the operand tiles to be there already
-  const bool pairs = nproj > 0 && fold_usable(c, ngw);
+  // on the tensor cores (the operand tiles of the cell's own order of G exist
+  // since its creation, so a caller with a scratch plan needs no allocation)
+  const bool pairs = nproj > 0 && c->proj.fold.ok;
   bool use_tc = false;
   if constexpr (sizeof(R) == 4)
-    use_tc = nproj > 0 && nl_tc_usable(c) && (!plan || nl_tc_have_tiles(c, pairs));
+    use_tc = nproj > 0 && nl_tc_usable(c);
   const bool fold = pairs && (use_tc || (sizeof(R) == 8 && !plan));
   float *tc_part = nullptr, *tc_wt = nullptr;
   int tc_split = 0;
@@ -840,8 +840,8 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
       if (!plan && fold) {
         cudaEvent_t e;
         timing_begin(c, kFamProj, &e);
-        const int rc = fold_project64(c, reinterpret_cast<const double2 *>(in), ld_in, nb,
-                                      reinterpret_cast<double2 *>(wp), false);
+        const int rc = fold_project64(c, reinterpret_cast<const double2 *>(in), ld_in, ngw,
+                                      nb, reinterpret_cast<double2 *>(wp), false);
         if (rc) return rc;
         timing_end(c, kFamProj, e);
         done = true;
@@ -1001,7 +1001,7 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
         if (!plan) {
           cudaEvent_t e;
           timing_begin(c, kFamBackproj, &e);
-          int rc = fold ? fold_backproject64(c, reinterpret_cast<const double2 *>(wp), nb,
+          int rc = fold ? fold_backproject64(c, reinterpret_cast<const double2 *>(wp), ngw, nb,
                                              reinterpret_cast<double2 *>(out), ld_out,
                                              pre ? a : 1.0)
                         : backproject_beta64(c, reinterpret_cast<const double2 *>(wp), ngw, nb,
@@ -1043,7 +1043,7 @@ int project_fp64(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, doub
   using R = double;
   const int nproj = c->proj.nproj;
   if (nproj <= 0 || nb <= 0) return PSPW_OK;
-  if (fold_usable(c, ngw)) return fold_project64(c, psi, ld, nb, P, true);
+  if (c->proj.fold.ok) return fold_project64(c, psi, ld, ngw, nb, P, true);
   ProjArg pa;
   pa.eigr = Prec<R>::eigr(c);
   pa.pkga = Prec<R>::pkga(c);

@@ -63,6 +63,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "fold.h"
 #include "nl_tc.h"
 #include "tc.cuh"
 
@@ -165,8 +166,9 @@ __device__ __forceinline__ void drain_bulk(Sync &sy, int issued, int nt) {
 __host__ __device__ constexpr int proj_slots(int npad) { return tmem_cols(npad) <= 64 ? 3 : 2; }
 constexpr int kStepG = 16;  // G per projection step
 
-// FOLD: ngw counts pairs (table `pair`), a raw row holds psi at +G and at -G,
-// and bit lm of `odd` marks the odd form factors.
+// FOLD: ngw counts pairs (table `pair`), a raw row holds psi at +G and at -G
+// (only the first npsi G of psi exist), and bit lm of `odd` marks the odd form
+// factors.
 __host__ __device__ constexpr int raw_row(bool fold) { return (fold ? 2 : 1) * (kStepG + 1); }
 
 // Raw slots in flight.  With one projector per atom a tile touches 65 bands and
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
                                                       const float *__restrict__ pkga, int nat,
                                                       int npad, int ksplit_g,
                                                       float *__restrict__ part, int *err,
-                                                      const int2 *__restrict__ pair,
+                                                      const int2 *__restrict__ pair, int npsi,
                                                       unsigned odd) {
   constexpr int per = 2 * L;
   constexpr int nbr_max = 127 / per + 2;  // bands a 128-row tile touches
@@ -296,7 +298,8 @@ __global__ void __launch_bounds__(kThreadsP) k_proj_tc(const float2 *__restrict_
       const int g0 = gb + kStepG * k;
       if constexpr (FOLD) {
         const int j = lane & (kStepG - 1);
-        const bool vx = pr.x >= 0, vy = pr.y >= 0;
+        // (x < y in every pair: without x there is no y either)
+        const bool vx = pr.x >= 0 && pr.x < npsi, vy = pr.y >= 0 && pr.y < npsi;
         const float2 *px = psi + (size_t)bfirst * ld + (vx ? pr.x : 0);
         const float2 *py = psi + (size_t)bfirst * ld + (vy ? pr.y : 0);
         for (int b = lane / kStepG; b < nbr; b += 32 / kStepG) {
@@ -595,7 +598,7 @@ __host__ __device__ constexpr int t2_col(int ncolN) { return (ncolN + 31) & ~31;
 template <int L, bool PRE>
 __global__ void __launch_bounds__(kThreads) k_backpair_tc(
     const float *__restrict__ etb, const float *__restrict__ wt, int nsa, int npair,
-    const int2 *__restrict__ pair, unsigned odd, int nb, int nbt, const float *__restrict__ pkga,
+    const int2 *__restrict__ pair, int ngw, unsigned odd, int nb, int nbt, const float *__restrict__ pkga,
     float2 *out, int ldo, const float2 *__restrict__ in, int ldi, const float2 *__restrict__ xm2,
     int ldx, float ca, float cb, float cg, int *err) {
   constexpr int per = 2 * L;
@@ -649,7 +652,8 @@ __global__ void __launch_bounds__(kThreads) k_backpair_tc(
     const uint32_t lane_base = sy.tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     const int j = gt * 128 + row;
     const int2 pr = j < npair ? pair[j] : make_int2(-1, -1);
-    const bool vp = pr.x >= 0, vm = pr.y >= 0;
+    // G of the call (its first ngw; x < y in every pair)
+    const bool vp = pr.x >= 0 && pr.x < ngw, vm = pr.y >= 0 && pr.y < ngw;
     const int nbh = nbt / 2;
     const int bstart = half * nbh;
     float pk[4] = {0.f, 0.f, 0.f, 0.f};
@@ -673,7 +677,7 @@ __global__ void __launch_bounds__(kThreads) k_backpair_tc(
         for (int q = 0; q < 2; q++) {
           const int g = q ? pr.y : pr.x;
           hv[i][q] = uv[i][q] = xv[i][q] = make_float2(0.f, 0.f);
-          if (on && g >= 0) {
+          if (on && (q ? vm : vp)) {
             hv[i][q] = out[bb * ldo + g];
             if (!PRE && cb != 0.f) uv[i][q] = in[bb * ldi + g];
             if (!PRE && cg != 0.f) xv[i][q] = xm2[bb * ldx + g];
@@ -948,7 +952,7 @@ int proj_splits(const Shape &s, int ngw, int nb, int *kg_out, bool fold) {
 }
 
 template <int L>
-int launch_project(pspw_cell *c, const Shape &s, const float2 *psi, int ld, int ngw, int nb,
+int launch_project(pspw_cell *c, const Shape &s, const float2 *psi, int ld, int nk, int ngw, int nb,
                    float *part, int nsplit, int kg, float *wt, const float *etp,
                    const float *pkga, const float *pw, bool fold, unsigned odd) {
   const int mt = (nb * s.per + 127) / 128;
@@ -957,7 +961,7 @@ int launch_project(pspw_cell *c, const Shape &s, const float2 *psi, int ld, int 
   int rc = smem_allow_max(kern);
   if (rc) return rc;
   kern<<<dim3(mt, nsplit), kThreadsP, smem, c->stream>>>(
-      psi, ld, ngw, nb, etp, pkga, s.nat, s.npad, kg, part, c->d_err, c->proj.fold.d_pair, odd);
+      psi, ld, nk, nb, etp, pkga, s.nat, s.npad, kg, part, c->d_err, c->proj.fold.d_pair, ngw, odd);
   const int nsa = fold ? (s.nat + 15) / 16 : s.nsa;
   const dim3 wgrid(((fold ? 8 : 4) * nsa + 31) / 32, s.nbtiles * s.nbt * L);
   auto wkern = fold ? k_proj_tc_wtiles<L, true> : k_proj_tc_wtiles<L, false>;
@@ -973,12 +977,12 @@ int launch_back(pspw_cell *c, const Shape &s, const float *wt, const float *etb,
                 int ldi, const float2 *xm2, int ldx, float a, float b, float g, bool pre, bool fold,
                 unsigned odd) {
   if (fold) {
-    const int npair = 8 * c->proj.fold.groups;
+    const int npair = 8 * fold_groups(c->proj.fold, ngw);
     auto kern = pre ? k_backpair_tc<L, true> : k_backpair_tc<L, false>;
     if (const int rc = smem_allow_max(kern)) return rc;
     const dim3 grid((npair + 127) / 128, s.nbtiles);
     kern<<<grid, kThreads, backpair_smem(s), c->stream>>>(
-        etb, wt, (s.nat + 15) / 16, npair, c->proj.fold.d_pair, odd, nb, s.nbt, pkga, out, ldo, in,
+        etb, wt, (s.nat + 15) / 16, npair, c->proj.fold.d_pair, ngw, odd, nb, s.nbt, pkga, out, ldo, in,
         ldi, xm2, ldx, a, b, g, c->d_err);
     c->kernel_launches++;
     PSPW_CUDA(cudaGetLastError());
@@ -1096,13 +1100,9 @@ int nl_tc_prepare(pspw_cell *c) {
   return nl_tc_ensure_tiles(c, c->proj.fold.ok);
 }
 
-bool nl_tc_have_tiles(const pspw_cell *c, bool fold) {
-  return fold ? c->proj.fold.etp != nullptr : c->proj.d_etp != nullptr;
-}
-
 int nl_tc_ensure_tiles(pspw_cell *c, bool fold) {
-  if (nl_tc_have_tiles(c, fold)) return PSPW_OK;
   Projectors &P = c->proj;
+  if (fold ? P.fold.etp : P.d_etp) return PSPW_OK;
   return fold ? nl_tc_pair_tiles(c) : nl_tc_build_tiles(c, P.d_eigr32, &P.d_etp, &P.d_etb);
 }
 
@@ -1118,8 +1118,8 @@ int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, f
   int ms = 1;
   for (const Group &g : groups_of(c->proj, c->basis.ngw)) {
     int kg = 0;
-    ms = std::max(ms, proj_splits(shape_of(g, nb), fold ? 8 * c->proj.fold.groups : ngw, nb, &kg,
-                                  fold));
+    ms = std::max(ms, proj_splits(shape_of(g, nb), fold ? 8 * fold_groups(c->proj.fold, ngw) : ngw,
+                                  nb, &kg, fold));
   }
   // the partial sums of any one species fit max_split x 2 nb nproj floats
   int rc = ws_reserve(c, kWsProjPart, sizeof(float) * (size_t)ms * 2 * nb * c->proj.nproj,
@@ -1134,7 +1134,7 @@ int nl_tc_reserve(pspw_cell *c, int ngw, int nb, float **part, int *max_split, f
 int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, float *part,
                   int max_split, float *wt, bool fold) {
   const Projectors &P = c->proj;
-  const int nk = fold ? 8 * P.fold.groups : ngw;  // pairs or G to sum over
+  const int nk = fold ? 8 * fold_groups(P.fold, ngw) : ngw;  // pairs or G to sum over
   const size_t cap = (size_t)std::max(1, max_split) * 2 * nb * P.nproj;  // floats of part
   size_t woff = 0;
   for (const Group &g : groups_of(P, c->basis.ngw, fold)) {
@@ -1154,19 +1154,19 @@ int nl_tc_project(pspw_cell *c, const float2 *psi, int ld, int ngw, int nb, floa
     int rc;
     switch (s.L) {
       case 1:
-        rc = launch_project<1>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+        rc = launch_project<1>(c, s, psi, ld, nk, ngw, nb, part, nsplit, kg, w,
                                 etp, pk, pw, fold, odd);
         break;
       case 2:
-        rc = launch_project<2>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+        rc = launch_project<2>(c, s, psi, ld, nk, ngw, nb, part, nsplit, kg, w,
                                 etp, pk, pw, fold, odd);
         break;
       case 3:
-        rc = launch_project<3>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+        rc = launch_project<3>(c, s, psi, ld, nk, ngw, nb, part, nsplit, kg, w,
                                 etp, pk, pw, fold, odd);
         break;
       default:
-        rc = launch_project<4>(c, s, psi, ld, nk, nb, part, nsplit, kg, w,
+        rc = launch_project<4>(c, s, psi, ld, nk, ngw, nb, part, nsplit, kg, w,
                                 etp, pk, pw, fold, odd);
     }
     if (rc) return rc;

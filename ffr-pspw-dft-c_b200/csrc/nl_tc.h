@@ -12,11 +12,9 @@ bool nl_tc_usable(const pspw_cell *c);
 
 // EIGR operand tiles of the cell's current G order, over pairs (fold; the
 // cell's fold must be ok) or over G.  A new cell gets those that its products
-// over the whole sphere use (nl_tc_prepare, no-op when the projectors do not
-// fit the kernels); the others, and the stick order's, are built when they
-// are first needed.
+// use (nl_tc_prepare, no-op when the projectors do not fit the kernels), the
+// stick order's are built when they are first needed.
 int nl_tc_prepare(pspw_cell *c);
-bool nl_tc_have_tiles(const pspw_cell *c, bool fold);
 int nl_tc_ensure_tiles(pspw_cell *c, bool fold);
 
 // Bytes of the projection operand tiles for nb bands.

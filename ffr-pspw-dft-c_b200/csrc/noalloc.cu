@@ -33,7 +33,6 @@
 
 #include "common.cuh"
 #include "engine.h"
-#include "fold.h"
 #include "nl_tc.h"
 
 #define PSPW_NOALLOC_SCRATCH_BYTES (16u << 20)
@@ -84,9 +83,9 @@ extern "C" int pspw_apply_ham_block_dev_noalloc(pspw_cell *c, int prec, const vo
   const size_t per_band = ((size_t)B.n3 * B.ncol + (size_t)B.n3 * B.n2 * B.nxa) * sc;
   const size_t slice = (size_t)nstates * c->proj.nproj * sc;  // one projection block
   // FP32 on the tensor-core path: the projections as operand tiles
-  const bool tc = prec == PSPW_PREC_F32 && nl_tc_usable(c) &&
-                  nl_tc_have_tiles(c, fold_usable(c, ngw));
-  const size_t wt_bytes = tc ? up256(nl_tc_wtile_bytes(c, nstates)) : 0;
+  // (the cell has the tiles since its creation)
+  const size_t wt_bytes =
+      prec == PSPW_PREC_F32 && nl_tc_usable(c) ? up256(nl_tc_wtile_bytes(c, nstates)) : 0;
   const size_t wp_bytes = up256(slice) + wt_bytes;
   // partial-sum slices: up to a quarter of the array, at least one
   int nsplit = slice ? (int)std::max<size_t>(1, std::min<size_t>(64, cap / 4 / slice)) : 1;
