@@ -784,18 +784,16 @@ int hpsi_apply(pspw_cell *c, const void *in_v, int ld_in, void *out_v, int ld_ou
   int tc_split = 0;
   // The projection reads psi only: it runs on the cell's second stream,
   // concurrently with the local part, and the back-projection waits for it
-  // (unless the cell's overlap mode is PSPW_OVERLAP_OFF; on Si64 the
-  // concurrent form is 6 % faster in FP32 and 8 % in FP64).  In the automatic
-  // mode small products (below 4 M elements of beta x bands) stay on the cell
-  // stream: such a call is bound by its launches, and the fork and join are
-  // four more driver calls.  Callers with a scratch plan, i.e. the
-  // allocation-free entry point, keep one stream.
+  // unless the cell's overlap mode is PSPW_OVERLAP_OFF.  The concurrent form is
+  // the faster one at every size: H*psi one call after the other on one cell of
+  // 8 atoms 26.6 against 40.0 us (FP32, 16 bands) and 23.6 against 31.6 (FP64,
+  // one band), since the projection's two kernels leave the chain of dependent
+  // ones; of 64 atoms 300 against 314 us (FP32, 128 bands).  Callers with a
+  // scratch plan, i.e. the allocation-free entry point, keep one stream.
   // c->stream is switched for the projection's launches and switched back
   // on every exit from this block.
   const cudaStream_t main_st = c->stream;
-  const bool worth = c->nl_overlap == PSPW_OVERLAP_ON ||
-                     (double)nproj * ngw * nb >= 4.0 * (1 << 20);
-  const bool overlap = c->nl_overlap != PSPW_OVERLAP_OFF && worth && nproj > 0 && !plan &&
+  const bool overlap = c->nl_overlap != PSPW_OVERLAP_OFF && nproj > 0 && !plan &&
                        c->stream2 != nullptr;
   struct StreamSwitch {
     pspw_cell *c;

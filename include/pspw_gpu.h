@@ -123,9 +123,8 @@ int pspw_cell_set_band_batch(pspw_cell *cell, int nbatch);
 int pspw_cell_set_nl_path(pspw_cell *cell, int path);
 
 /* Whether the projection of H*psi runs on the cell's second stream,
- * concurrently with the FFT passes (ON), or on the cell stream (OFF); AUTO
- * takes the second stream where the products are large enough to gain from
- * it; no reference counterpart.  Results do not depend on it (the
+ * concurrently with the FFT passes (AUTO, ON), or after them on the cell
+ * stream (OFF); no reference counterpart.  Results do not depend on it (the
  * same kernels run in the same order of arithmetic).  The allocation-free
  * entry point always keeps one stream. */
 #define PSPW_OVERLAP_AUTO 0
