@@ -939,12 +939,19 @@ int sm_count() {
   return n;
 }
 
-// splits of the projection's K range: enough blocks to fill the GPU once
+// Splits of the projection's K range: enough blocks to fill the GPU once, of
+// 64 units (G, or pairs with `fold`) or more.  A slice of 64 pairs has twice
+// the G, so a small sphere would keep half the blocks it had over G: down to
+// 32 pairs each, up to one block per SM (Si8, 36^3, 16 bands: the FP32 filter
+// of 8 applications 241 -> 228 us).  Slices of 32 beyond that cost more in the
+// reduction than they save (Si64, one band: H*psi 32 -> 38 us with 296 slices).
 int proj_splits(const Shape &s, int ngw, int nb, int *kg_out, bool fold) {
   const int mt = (nb * s.per + 127) / 128;
   const int smem = proj_smem(s, fold);
   const int per_sm = std::max(1, std::min(233472 / (smem + 1024), 512 / proj_tmem_cols(s)));
-  int nsplit = std::max(1, std::min((ngw + 63) / 64, per_sm * sm_count() / mt));
+  int most = (ngw + 63) / 64;
+  if (fold) most = std::max(most, std::min((ngw + 31) / 32, sm_count() / mt));
+  int nsplit = std::max(1, std::min(most, per_sm * sm_count() / mt));
   int kg = (ngw + nsplit - 1) / nsplit;
   kg = (kg + kStepG - 1) / kStepG * kStepG;
   *kg_out = kg;
