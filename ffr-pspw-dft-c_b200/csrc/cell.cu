@@ -531,7 +531,7 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
       cudaHostGetDevicePointer((void **)&c->d_err, c->h_err, 0) != cudaSuccess)
     return bail(fail(PSPW_ERR_OOM, "cell_create: error word"));
   *c->h_err = 0;
-  if ((rc = pspw::fold_prepare(c, gi1.data(), gi2.data(), gi3.data(), order.data())))
+  if ((rc = pspw::fold_prepare(c, col_x, col_y, col_of_xy, col_start, sg_z, order)))
     return bail(rc);
   if ((rc = pspw::nl_tc_prepare(c))) return bail(rc);
   *out = c;

@@ -85,6 +85,14 @@ __global__ void k_fold_check(const int2 *__restrict__ pair, int npair, int ngw, 
   }
 }
 
+// odd[p]: the form factor of projector p is not even
+__global__ void k_fold_odd(const int *__restrict__ flags, const int *__restrict__ psp,
+                           const int *__restrict__ plm, int nproj,
+                           unsigned char *__restrict__ odd) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < nproj) odd[p] = !flags[1 + 2 * (4 * psp[p] + plm[p])];
+}
+
 // B: 16 rows per group (8 u rows, then 8 V rows), columns p = blockIdx.y
 __global__ void k_fold_build(const int2 *__restrict__ pair, int groups, int ngw,
                              const double2 *__restrict__ eigr, const double *__restrict__ pkga,
@@ -578,91 +586,81 @@ int tile_bands(int nb) {
 
 }  // namespace
 
-int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, const int *order) {
+int fold_prepare(pspw_cell *c, const std::vector<int> &col_x, const std::vector<int> &col_y,
+                 const std::vector<int> &col_of_xy, const std::vector<int> &col_start,
+                 const std::vector<int> &sg_z, const std::vector<int> &order) {
   const Basis &B = c->basis;
   Projectors &P = c->proj;
   if (P.nproj <= 0) return PSPW_OK;
   const int ngw = B.ngw;
-  // the partner of G sits at the negated grid index
-  std::vector<int> at(B.nnr, -1), partner(ngw);
-  auto idx = [&](int a, int b, int d) { return ((size_t)d * B.n2 + b) * B.n1 + a; };
-  for (int g = 0; g < ngw; g++) {
-    int &s = at[idx(gi1[g], gi2[g], gi3[g])];
-    if (s >= 0) return PSPW_OK;  // two G on one grid point
-    s = g;
+  // The partner of G sits at the negated grid index: in the stick (-x, -y), whose
+  // z's are the negated ones of G's stick in reverse, after z = 0.  partner[k]:
+  // stick-list position of the partner of position k.
+  std::vector<int> partner(ngw);
+  for (int k = 0; k < B.ncol; k++) {
+    const int x = col_x[k], y = col_y[k], k0 = col_start[k], m = col_start[k + 1] - k0;
+    const int q = col_of_xy[(x ? B.n1 - x : 0) + (size_t)B.n1 * (y ? B.n2 - y : 0)];
+    if (q < 0 || col_start[q + 1] - col_start[q] != m) return PSPW_OK;
+    const int zero = sg_z[k0] == 0;
+    for (int i = 0; i < m; i++) {
+      const int z = sg_z[k0 + i], j = col_start[q] + (i < zero ? 0 : m - 1 - i + zero);
+      if (i > 0 && z == sg_z[k0 + i - 1]) return PSPW_OK;  // two G on one grid point
+      if (sg_z[j] != (z ? B.n3 - z : 0)) return PSPW_OK;
+      partner[k0 + i] = j;
+    }
   }
-  for (int g = 0; g < ngw; g++) {
-    partner[g] = at[idx((B.n1 - gi1[g]) % B.n1, (B.n2 - gi2[g]) % B.n2, (B.n3 - gi3[g]) % B.n3)];
-    if (partner[g] < 0) return PSPW_OK;
-  }
-  std::vector<int> pos(ngw);
-  for (int k = 0; k < ngw; k++) pos[order[k]] = k;
-  const int npair = [&] {
-    int n = 0;
-    for (int g = 0; g < ngw; g++) n += partner[g] >= g;
-    return n;
-  }();
+  int npair = 0;
+  for (int k = 0; k < ngw; k++) npair += partner[k] >= k;
   const int groups = (npair + kGroup - 1) / kGroup;
-  std::vector<int2> nat_pairs, stick_pairs;
-  nat_pairs.reserve((size_t)groups * kGroup);
-  stick_pairs.reserve((size_t)groups * kGroup);
-  for (int g = 0; g < ngw; g++) {
-    if (partner[g] >= g) nat_pairs.push_back(make_int2(g, partner[g] == g ? -1 : partner[g]));
-    const int q = pos[partner[order[g]]];  // stick position g's partner
-    if (q >= g) stick_pairs.push_back(make_int2(g, q == g ? -1 : q));
+  // one allocation and one copy: the pair tables of both orders, the check's
+  // flags, and the odd marks (device only)
+  const size_t np = (size_t)groups * kGroup, nflags = 1 + 8 * (size_t)P.nsp;
+  std::vector<int2> host(2 * np + (nflags + 1) / 2, make_int2(-1, -1));
+  int2 *nat = host.data(), *stick = nat + np;
+  int *flags = reinterpret_cast<int *>(stick + np);
+  std::fill(flags, flags + nflags, 1);
+  std::vector<int> nat_partner(ngw);
+  for (int k = 0; k < ngw; k++) {
+    const int q = partner[k];
+    nat_partner[order[k]] = order[q];
+    if (q >= k) *stick++ = make_int2(k, q == k ? -1 : q);
   }
-  nat_pairs.resize((size_t)groups * kGroup, make_int2(-1, -1));
-  stick_pairs.resize((size_t)groups * kGroup, make_int2(-1, -1));
+  for (int g = 0; g < ngw; g++)
+    if (nat_partner[g] >= g) *nat++ = make_int2(g, nat_partner[g] == g ? -1 : nat_partner[g]);
   Fold &f = P.fold, &fs = c->stick.fold;
   f.groups = fs.groups = groups;
   for (int g = 0; g < groups; g++) {  // (the last group has a pair too)
-    f.first.push_back(nat_pairs[(size_t)g * kGroup].x);
-    fs.first.push_back(stick_pairs[(size_t)g * kGroup].x);
+    f.first.push_back(host[(size_t)g * kGroup].x);
+    fs.first.push_back(host[np + (size_t)g * kGroup].x);
   }
-  std::vector<int> flags(1 + 8 * (size_t)P.nsp, 1);
-  // one allocation: both pair tables, the check's flags, the odd marks
-  const size_t np = nat_pairs.size(), bytes = sizeof(int2) * np;
-  if (cudaMalloc(&P.fold_mem, 2 * bytes + flags.size() * sizeof(int) + P.nproj) != cudaSuccess)
+  if (cudaMalloc(&P.fold_mem, sizeof(int2) * host.size() + P.nproj) != cudaSuccess)
     return fail(PSPW_ERR_OOM, "G pairs");
   f.d_pair = static_cast<int2 *>(P.fold_mem);
   fs.d_pair = f.d_pair + np;
   int *d_flags = reinterpret_cast<int *>(fs.d_pair + np);
-  P.d_odd = reinterpret_cast<unsigned char *>(d_flags + flags.size());
-  std::vector<unsigned char> odd;
-  auto run = [&]() -> int {
-    cudaStream_t st = c->stream;
-    PSPW_CUDA(cudaMemcpyAsync(f.d_pair, nat_pairs.data(), bytes, cudaMemcpyHostToDevice, st));
-    PSPW_CUDA(cudaMemcpyAsync(fs.d_pair, stick_pairs.data(), bytes, cudaMemcpyHostToDevice, st));
-    PSPW_CUDA(cudaMemcpyAsync(d_flags, flags.data(), flags.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, st));
-    const long long n = (long long)(P.nat + P.nsp) * npair;
-    k_fold_check<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
-        f.d_pair, npair, ngw, P.nat, P.nsp, P.d_eigr64, P.d_pkga64, d_flags);
-    c->kernel_launches++;
-    PSPW_CUDA(cudaGetLastError());
-    PSPW_CUDA(cudaMemcpyAsync(flags.data(), d_flags, flags.size() * sizeof(int),
-                              cudaMemcpyDeviceToHost, st));
-    PSPW_CUDA(cudaStreamSynchronize(st));
-    bool ok = flags[0] != 0;
-    for (int s = 0; s < P.nsp && ok; s++)
-      for (int lm = 0; lm < P.sp_lm[s]; lm++)
-        if (P.sp_na[s] > 0)
-          ok = ok && (flags[1 + 2 * (4 * s + lm)] || flags[2 + 2 * (4 * s + lm)]);
-    P.sp_odd.assign(P.nsp, 0u);
-    for (int s = 0; s < P.nsp; s++)
-      for (int lm = 0; lm < 4; lm++)
-        if (!flags[1 + 2 * (4 * s + lm)]) P.sp_odd[s] |= 1u << lm;
-    for (int s = 0; s < P.nsp; s++)
-      for (int a = 0; a < P.sp_na[s]; a++)
-        for (int lm = 0; lm < P.sp_lm[s]; lm++) odd.push_back(!flags[1 + 2 * (4 * s + lm)]);
-    if (ok) {
-      PSPW_CUDA(cudaMemcpyAsync(P.d_odd, odd.data(), odd.size(), cudaMemcpyHostToDevice, st));
-      PSPW_CUDA(cudaStreamSynchronize(st));
-    }
-    f.ok = fs.ok = ok;
-    return PSPW_OK;
-  };
-  return run();
+  P.d_odd = reinterpret_cast<unsigned char *>(f.d_pair + host.size());
+  cudaStream_t st = c->stream;
+  PSPW_CUDA(cudaMemcpyAsync(P.fold_mem, host.data(), sizeof(int2) * host.size(),
+                            cudaMemcpyHostToDevice, st));
+  const long long n = (long long)(P.nat + P.nsp) * npair;
+  k_fold_check<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
+      f.d_pair, npair, ngw, P.nat, P.nsp, P.d_eigr64, P.d_pkga64, d_flags);
+  k_fold_odd<<<(P.nproj + 255) / 256, 256, 0, st>>>(d_flags, P.d_psp, P.d_plm, P.nproj, P.d_odd);
+  c->kernel_launches += 2;
+  PSPW_CUDA(cudaGetLastError());
+  PSPW_CUDA(cudaMemcpyAsync(flags, d_flags, nflags * sizeof(int), cudaMemcpyDeviceToHost, st));
+  PSPW_CUDA(cudaStreamSynchronize(st));
+  bool ok = flags[0] != 0;
+  for (int s = 0; s < P.nsp && ok; s++)
+    for (int lm = 0; lm < P.sp_lm[s]; lm++)
+      if (P.sp_na[s] > 0)
+        ok = ok && (flags[1 + 2 * (4 * s + lm)] || flags[2 + 2 * (4 * s + lm)]);
+  P.sp_odd.assign(P.nsp, 0u);
+  for (int s = 0; s < P.nsp; s++)
+    for (int lm = 0; lm < 4; lm++)
+      if (!flags[1 + 2 * (4 * s + lm)]) P.sp_odd[s] |= 1u << lm;
+  f.ok = fs.ok = ok;
+  return PSPW_OK;
 }
 
 int fold_groups(const Fold &f, int ngw) {

@@ -1,16 +1,21 @@
 // FP64 projector products over pairs (+G, -G) (fold.cu).
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 #include "engine.h"
 
 namespace pspw {
 
-// Finds the pairs of a cell's sphere from its grid indices (gi1, gi2, gi3 of
-// each G, `order` = the stick lists' G order) and checks on the device that
-// EIGR and PKG_A have the symmetry, for every value.  Called once at cell
-// creation, after the projector arrays; leaves fold.ok false otherwise.
-int fold_prepare(pspw_cell *c, const int *gi1, const int *gi2, const int *gi3, const int *order);
+// Finds the pairs of a cell's sphere from its stick lists (cell_create's:
+// sticks in ascending (y, x), their G in ascending z, `order` the G of each
+// position) and checks on the device that EIGR and PKG_A have the symmetry, for
+// every value.  Called once at cell creation, after the projector arrays;
+// leaves fold.ok false otherwise.
+int fold_prepare(pspw_cell *c, const std::vector<int> &col_x, const std::vector<int> &col_y,
+                 const std::vector<int> &col_of_xy, const std::vector<int> &col_start,
+                 const std::vector<int> &sg_z, const std::vector<int> &order);
 
 // Groups that hold a pair with one of the first ngw G (pairs are in ascending
 // order of their first G).
