@@ -24,7 +24,7 @@ Split split_for(int n) {
   for (int b = 1; b <= 61; b++) {
     if (n % b || !radix(b)) continue;
     const int a = n / b;
-    if (a > 16 || (b <= 16 && a < b && n / a != b)) continue;
+    if (a > 16) continue;
     const int mx = std::max(a, b);
     // ties: the larger factor as the block factor (contiguous elements)
     if (mx < best_max || (mx == best_max && b <= 16 && a > best.a)) {

@@ -895,26 +895,25 @@ __global__ void __launch_bounds__(32 * kBTWarps) k_back_tr(const double2 *__rest
 // is not positive, stat[1] = max |U_kk| / min |U_kk|.  Works on L packed in
 // shared memory; k_tri_inv then forms U^-1 on many blocks.
 //
-// mode kCholScaled: the factor is that of D G D with D = diag(G)^-1/2, the
-// Gram matrix of the columns scaled to unit norm, and scale[i] = D_ii (a
-// column that is zero, or whose squared norm is too small or large to hold
-// its digits, counts as a failed pivot).
-// mode kCholNear: when max |G - I| < 1e-9 no factorisation is needed: stat[1]
-// = -1 and k_tri_inv takes U^-1 to first order in G - I, whose square is
-// below n * 1e-18.  The second pass of CholeskyQR2 ends so unless the block
+// Without `near` the factor is that of D G D with D = diag(G)^-1/2, the Gram
+// matrix of the columns scaled to unit norm, and scale[i] = D_ii (a column
+// that is zero, or whose squared norm is too small or large to hold its
+// digits, counts as a failed pivot).
+// With `near`, G is factored as it is, or not at all when max |G - I| < 1e-9:
+// then stat[1] = -1 and k_tri_inv takes U^-1 to first order in G - I, whose
+// square is below n * 1e-18.  The second pass of CholeskyQR2 ends so unless the block
 // was ill-conditioned; its factorisation and inverse took 165 + 33 us at
 // order 146, this check 6 us.
-constexpr int kCholPlain = 0, kCholScaled = 1, kCholNear = 2;
 __global__ void __launch_bounds__(kT1, 1)
     k_chol_inv(const double2 *__restrict__ G, int ldg, int n, double2 *__restrict__ Lg,
-               double *__restrict__ stat, int mode, double *__restrict__ scale) {
+               double *__restrict__ stat, bool near, double *__restrict__ scale) {
   extern __shared__ double2 L[];
   __shared__ int s_failed;
   __shared__ double s_d[kHeevMax];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   if (tid == 0) s_failed = 0;
   __syncthreads();
-  if (mode == kCholNear) {
+  if (near) {
     int far = 0;
     for (int i = warp; i < n; i += nw)
       for (int j = lane; j <= i; j += 32) {
@@ -930,7 +929,7 @@ __global__ void __launch_bounds__(kT1, 1)
       return;
     }
   }
-  if (mode == kCholScaled) {
+  if (!near) {
     for (int i = tid; i < n; i += blockDim.x) {
       const double g = G[i + (size_t)i * ldg].x;
       const bool ok = g > 1e-200 && g < 1e200;
@@ -943,7 +942,7 @@ __global__ void __launch_bounds__(kT1, 1)
   for (int i = warp; i < n; i += nw)
     for (int j = lane; j <= i; j += 32) {
       double2 g = cconj(G[j + (size_t)i * ldg]);
-      if (mode == kCholScaled) {
+      if (!near) {
         g = i == j ? make_double2(1.0, 0.0)
                    : make_double2(s_d[i] * s_d[j] * g.x, s_d[i] * s_d[j] * g.y);
       }
@@ -1190,10 +1189,9 @@ int dev_chol_inv_upper(pspw_cell *c, const double2 *G, int ldg, int n, double2 *
   int rc;
   if ((rc = ws_reserve(c, kWsChol, sizeof(double2) * (size_t)np, (void **)&Lg))) return rc;
   if ((rc = smem_allow_max(k_chol_inv)) || (rc = smem_allow_max(k_tri_inv))) return rc;
-  const int mode = near_identity ? kCholNear : (scale ? kCholScaled : kCholPlain);
-  k_chol_inv<<<1, kT1, smem, c->stream>>>(G, ldg, n, Lg, stat, mode, scale);
+  k_chol_inv<<<1, kT1, smem, c->stream>>>(G, ldg, n, Lg, stat, near_identity, scale);
   k_tri_inv<<<(n + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, smem, c->stream>>>(
-      Lg, n, Uinv, ldu, stat, mode == kCholScaled ? scale : nullptr, G, ldg);
+      Lg, n, Uinv, ldu, stat, near_identity ? nullptr : scale, G, ldg);
   c->kernel_launches += 2;
   PSPW_CUDA(cudaGetLastError());
   return PSPW_OK;

@@ -29,11 +29,11 @@ int dev_heev_small(pspw_cell *c, double2 *A, int lda, double *w, int n, void *wo
 // stat[0] (device) <- 0, or k + 1 if the k-th pivot is not positive;
 // stat[1] <- max |U_kk| / min |U_kk|.  n <= kHeevMax: the factor in one
 // block, the inverse on ceil(n / 4) blocks (one warp per column); Uinv is
-// left untouched when the factorisation fails.  With scale (device, n), the
-// factor is that of the columns' Gram matrix scaled to a unit diagonal and
-// Uinv carries the scaling, so X Uinv orthonormalises the X that G came from.
-// With near_identity, G within 1e-9 of the identity is inverted to first
-// order and stat[1] <- -1.
+// left untouched when the factorisation fails.  The factor is that of the
+// columns' Gram matrix scaled to a unit diagonal and Uinv carries the scaling
+// (kept in scale, device, n), so X Uinv orthonormalises the X that G came from.
+// With near_identity there is no scaling, and G within 1e-9 of the identity is
+// inverted to first order, stat[1] <- -1.
 int dev_chol_inv_upper(pspw_cell *c, const double2 *G, int ldg, int n, double2 *Uinv, int ldu,
                        double *stat, double *scale, bool near_identity);
 
