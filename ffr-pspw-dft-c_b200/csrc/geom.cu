@@ -819,10 +819,11 @@ struct GlibcRand {
   uint32_t s[31];
   int f = 3, b = 0;
   explicit GlibcRand(unsigned seed) {
-    int64_t r = seed ? seed : 1;
+    int64_t r = seed ? (int32_t)seed : 1;  // the library's table is signed
     for (int i = 0; i < 31; i++) {
       s[i] = (uint32_t)r;
       r = 16807 * r % 2147483647;
+      if (r < 0) r += 2147483647;
     }
     for (int i = 0; i < 310; i++) step();
   }
