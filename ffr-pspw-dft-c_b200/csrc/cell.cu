@@ -240,8 +240,7 @@ int pspw_cell_destroy(pspw_cell *c) {
   void *ptrs[] = {B.d_col_start, B.d_sg_ig, B.d_sg_z, B.d_sg_col, B.d_sg_off, B.d_col_of_xy,
                   B.d_xa_list,
                   B.d_xa_of_x, B.d_kin64, B.d_kin32, B.d_xkg64, c->proj.d_eigr64, c->proj.d_eigr32,
-                  c->proj.d_pkga64, c->proj.d_pkga32, c->proj.d_patom, c->proj.d_psp,
-                  c->proj.d_plm, c->proj.d_pw64, c->proj.d_pw32, c->d_veff64, c->d_veff32,
+                  c->proj.d_pkga64, c->proj.d_pkga32, c->proj.d_pw64, c->d_veff64, c->d_veff32,
                   B.d_col_x, c->d_vperm64, c->proj.d_etp, c->proj.d_etb, B.d_wgrid, c->proj.d_beta64,
                   c->stick.sg_ig, c->stick.kin64, c->stick.kin32, c->stick.eigr64,
                   c->stick.eigr32, c->stick.pkga64, c->stick.pkga32, c->stick.etp,
@@ -519,10 +518,20 @@ int cell_create(pspw_cell **out, int device, int nr1, int nr2, int nr3, int ngw,
                (rc = upload(&P.d_pkga64, k64)) || (rc = upload(&P.d_pkga32, k32))) {
       return bail(rc);
     }
-    if ((rc = upload(&P.d_patom, patom)) || (rc = upload(&P.d_psp, psp)) ||
-        (rc = upload(&P.d_plm, plm)) || (rc = upload(&P.d_pw64, pw64)) ||
-        (rc = upload(&P.d_pw32, pw32)))
-      return bail(rc);
+    // one table and one allocation: WNL in both precisions, then the indices
+    std::vector<double> tab(pw64);
+    tab.resize(3 * (size_t)nproj);
+    char *t = reinterpret_cast<char *>(tab.data() + nproj);
+    const size_t n4 = 4 * (size_t)nproj;
+    std::memcpy(t, pw32.data(), n4);
+    std::memcpy(t + n4, patom.data(), n4);
+    std::memcpy(t + 2 * n4, psp.data(), n4);
+    std::memcpy(t + 3 * n4, plm.data(), n4);
+    if ((rc = upload(&P.d_pw64, tab))) return bail(rc);
+    P.d_pw32 = reinterpret_cast<float *>(P.d_pw64 + nproj);
+    P.d_patom = reinterpret_cast<int *>(P.d_pw32 + nproj);
+    P.d_psp = P.d_patom + nproj;
+    P.d_plm = P.d_psp + nproj;
   }
   if (cudaMalloc(&c->d_veff64, (size_t)B.nnr * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->d_veff32, (size_t)B.nnr * sizeof(float)) != cudaSuccess)
