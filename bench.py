@@ -996,9 +996,9 @@ def run_engine(args, rank, world, local_rank):
     sc, sr = (16, 8) if fp64 else (8, 4)
     calls = args.steps * DEGREE
     names = {3: "k_sticks_inv", 5: "k_plane", 7: "k_sticks_fwd", 8: "k_proj_tc(+k_proj_tc_wtiles)",
-             9: "k_backproj_tc"}
+             9: "k_backpair_tc"}
     if fp64:
-        names.update({8: "k_proj(+k_proj_reduce)", 9: "k_backproj"})
+        names.update({8: "k_fold_proj(+k_fold_reduce)", 9: "k_fold_back"})
     fam_ms = {f: fam[f][0] for f in fam if fam[f][1] > 0}
     nproj = sizes["nproj"]
     alg_bytes = {  # per H*psi call

@@ -102,8 +102,7 @@ struct Projectors {
   double *d_pw64 = nullptr;  // [nproj] WNL(species, lm)
   float *d_pw32 = nullptr;
   // EIGR split into TF32 hi/lo operand tiles of the tensor-core projector
-  // GEMMs that run over G (nl_tc.cu; built when a product needs them, the
-  // pair tiles of `fold` otherwise)
+  // GEMMs over G (nl_tc.cu), for cells without the pair tiles of `fold`
   float *d_etp = nullptr;  // projection: per 8 G, [npad atoms x 16] hi then lo
   float *d_etb = nullptr;  // back-projection: per (128 G, 8 atoms), [128 x 16] hi then lo
   // (both hold one block of tiles per species with projectors, species in order)

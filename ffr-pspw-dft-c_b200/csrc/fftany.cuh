@@ -17,18 +17,20 @@
 // plus the run-time strides (one integer add per element).  The generic
 // five-pass path it replaces moved every plane through L2 twice, divided
 // integers per element, and took primes as direct sums on a local-memory
-// array.  Block H*psi, before -> with these kernels: 50 x 64 x 45, 93 bands
-// FP32 383 -> 124 us; 74^3, 32 bands FP64 10.5 -> 0.58 ms; six cells of
-// 30..60 points per axis in one batch, FP32 2.23 -> 0.72 ms.  Per point of a
-// plane 6.9 ps (50 x 64, FP32) against 4.9 ps of the compiled 64 x 64.
+// array.  Block H*psi, before -> with these kernels (-> now, with the pair
+// projectors too): 50 x 64 x 45, 93 bands FP32 383 -> 124 -> 112 us; 74^3, 32
+// bands FP64 10.5 -> 0.58 -> 0.53 ms; six cells of 30..60 points per axis in one
+// batch, FP32 2.23 -> 0.72 -> 0.63 ms.  Per point of a plane 6.9 ps (50 x 64,
+// FP32) against 4.9 ps of the compiled 64 x 64.
 //
 // Primes above 13 hold the item's (p - 1) / 2 symmetric pairs in registers
 // and loop over the output pairs, with the cosines and sines broadcast from
 // a shared-memory table: (p - 1)^2 multiply-adds per transform.  Kernels are
 // compiled per class of the largest factor, so small factors do not pay for
-// the registers of large primes (one class for all primes: a class of its own
-// for p <= 37 gained nothing, since 255 FP64 registers at 128 threads hold
-// p = 37 without spills and 168 at 160 threads do not, 727 against 579 us).
+// the registers of large primes.  One class holds all primes, 128 threads of 255
+// registers in FP64 (the largest primes spill 388 bytes of stores in the plane
+// kernel, 228 in the density's; FP32 takes 184 and none): a class of its own for
+// p <= 37 at 160 threads and 168 registers spilled more, 727 against 579 us.
 #pragma once
 
 #include <algorithm>
@@ -504,7 +506,8 @@ int any_plane(const Basis &B, const FastGeo &g, cudaStream_t st, int nbb, const 
       if (B.n1 * B.n2 < 6000) {
         // blocks of 256 threads held to the registers of five (FP32: 63 -> 48)
         // or three (FP64: 118 -> 80) per SM; shared memory leaves room for
-        // eight and four (six FP32 cells in a batch 683 -> 631 us)
+        // eight and four (six FP32 cells in a batch 683 -> 631 us, 44 bytes of
+        // spilled stores included)
         auto k = k_plane_any<CLS, 256, f32 ? 5 : 3, T, R>;
         if (const int rc = smem_allow_max(k)) return rc;
         k<<<grid, 256, sm, st>>>(g, p, B.n3, wx, wy, vperm, S);

@@ -169,10 +169,12 @@ constexpr size_t plane_smem() {
   return sizeof(T) * ((size_t)NY * PlaneCfg<NX, NY>::LS + NX + NY) + sizeof(int) * NX;
 }
 
-// FP64 planes of 60 and 64 points per axis, which take 100 and 88 registers
-// (two blocks per SM), are held to the registers of three, for which shared
-// memory has room (150 bands: 256 -> 232 and 246 -> 225 us).  All others leave
-// it to the compiler (0): a bound they do not need costs them 5 to 10 %.
+// FP64 planes of 60 points per axis or more take more than the 80 registers of
+// three blocks per SM (60: 100, 64: 88).  Where shared memory has room for three
+// (up to 64) they are held to 80 (150 bands: 256 -> 232 and 246 -> 225 us).
+// Smaller planes take 80 or fewer by themselves, larger ones fit twice at most:
+// all those leave it to the compiler (0), since a bound they do not need costs
+// them 5 to 10 %.
 template <int NX, int NY, typename T>
 constexpr int plane_min_blocks() {
   return sizeof(T) == 16 && PlaneCfg<NX, NY>::NT == 256 && NX >= 60 &&

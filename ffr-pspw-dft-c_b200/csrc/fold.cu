@@ -30,9 +30,10 @@
 // rows of one group, so a thread holds A and Q of its pairs and writes both
 // G's.  What bounds both at many bands: the FP64 tensor pipe, at half the
 // complex GEMM's operations.  Si64, 144 bands: 303 + 276 -> 162 + 145 us
-// (projection, back-projection; 64 x 32 tiles); Si216, 512 bands: the
-// back-projection 4.6 ms, 31 TFLOP/s.  Whole calls: FP64 filter of Si64 9.51 ->
-// 7.36 ms, H*psi of Si216 24.7 -> 17.2 ms.  The error of the projections
+// (projection, back-projection; 64 x 48 tiles, DMMA pipe 70 and 62 % busy);
+// Si216, 512 bands: the back-projection 4.6 ms, 31 TFLOP/s.  Whole calls: FP64
+// filter of Si64 9.51 -> 7.36 ms by these products alone, H*psi of Si216 24.7 ->
+// 17.2 ms.  The error of the projections
 // against extended precision is unchanged (Si216: 9.0e-15 both ways).  One
 // band: matrix-vector kernels, bound by reading B once from L2 or HBM.
 #include <cuda_runtime.h>
@@ -118,8 +119,9 @@ __global__ void k_fold_build(const int2 *__restrict__ pair, int groups, int ngw,
 // Tiles of (32 WM) x (16 WN) outputs, warps of 32 x 16; WM 1 or 2, WN 1 to 4.
 template <int WM, int WN>
 struct Ft {
-  // two ring slots for the 64 x 32 tile: with three, shared memory held 3 of
-  // the 4 blocks per SM that registers allow
+  // two ring slots for the tiles of four warps: with three, shared memory held
+  // 3 of the 4 blocks per SM that registers allow (64 x 32; the 32 x 64 tile
+  // measures the same either way, 94.3 and 94.2 us at 128 bands of Si8)
   static constexpr int BM = 32 * WM, BN = 16 * WN, BK = 16, STAGES = WM * WN == 4 ? 2 : 3;
   static constexpr int THREADS = 32 * WM * WN;
   // padded so that the fragment loads of a half warp (8-byte B) or a quarter
@@ -677,8 +679,9 @@ int fold_project64(pspw_cell *c, const double2 *psi, int ld, int ngw, int nb, do
   if (nb == 1) {
     // slices of 64 groups (two rounds of 256 threads) or more, four blocks per
     // SM; up to 512 groups (a sphere of 8192 G) one slice, which needs no
-    // reduction launch: such a call is bound by its launches (Si8, 369 groups:
-    // a call of 21 us with a reduction, 19 us without)
+    // reduction launch.  Calls of 256 projectors, one slice against several:
+    // 379 groups 30.8 / 35.6 us, 584 33.8 / 37.1, 696 35.8 / 34.4, 1490 58.6 /
+    // 53.2; of 32 projectors, 369 groups 22.5 / 23.6
     const int pt = (P.nproj + kVP - 1) / kVP;
     const int used = fold_groups(f, ngw);
     int nsplit = used <= 512 ? 1
